@@ -477,9 +477,9 @@ VH_HD inline bool c2p_ift_vjp(const DevCfg& C, const double* Tt, const double* p
 template <class R>
 VH_HD inline void obs_cell(const DevCfg& C, R e, R u1, R u2, R p1, R p2, double& num, double& den) {
   const R P = eos_P<R>(C, e), ep = e + P;
-  const double txx = (double)(ep * u1 * u1 + P + p1), tyy = (double)(ep * u2 * u2 + P + p2);
-  num = txx - tyy;
-  den = txx + tyy;
+  // T^xx - T^yy without the pressure that cancels in it
+  num = (double)(ep * (u1 * u1 - u2 * u2) + (p1 - p2));
+  den = (double)(ep * (u1 * u1 + u2 * u2) + (R)2 * P + (p1 + p2));
 }
 // adjoint of eps_p = N/D at one cell: returns eb, u1b, u2b, p1b, p2b
 template <class R>

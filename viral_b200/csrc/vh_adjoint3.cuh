@@ -94,7 +94,7 @@ VH_HD inline void pi_full_bar(const R pib[4][4], R* pb, PiDep<R>& db) {
 }
 
 // ---------------------------------------------------------- flux quantities
-// The flux quantities of one cell along DIR, as k_dir's cell_terms forms them
+// The flux quantities of one cell along DIR, as the sweep forms them (cell_flux)
 // (NEWEST5/hydroKT.h:16-83, 161-245): with a = DIR + 1,
 //   F^mu = tau (pi^{a mu} + P g^{a mu}-part + u^a u^mu (e + P)), mu = 0..3
 //   F^{4+l} = f_a pi_l u^a / u^tau,  speed = f_a u^a / u^tau (interior only)

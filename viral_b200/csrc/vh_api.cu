@@ -119,8 +119,10 @@ extern "C" int vh_create(const vh_config* cfg, vh_handle** out) {
   if ((e = cudaMalloc(&h->part, sizeof(double) * 8 * h->part_blocks + 32)) != cudaSuccess) return bail(e, "reduce");
   if ((e = cudaMemset(h->status, 0, sizeof(unsigned int))) != cudaSuccess) return bail(e, "status");
   if ((e = cudaMemset(h->iters, 0, sizeof(unsigned long long))) != cudaSuccess) return bail(e, "iters");
-  set_ptrs(h->pd, h->state, C.n, h->status, h->iters);
-  set_ptrs(h->pf, h->state, C.n, h->status, h->iters);
+  // the staging buffer is idle during a stage: its 18 arrays take the flux
+  // divergence along y and eta
+  set_ptrs(h->pd, h->state, h->stage, C.n, h->status, h->iters);
+  set_ptrs(h->pf, h->state, h->stage, C.n, h->status, h->iters);
   if ((h->mixed ? set_smem_attrs<float>(h) : set_smem_attrs<double>(h)) != VH_OK) {
     g_create_err = "vh_create: " + h->err;
     vh_destroy(h);
@@ -243,7 +245,7 @@ static int timed_steps(vh_handle* h, const DevPtrs<R>& P, int nsteps, double* ou
     for (int stage = 0; stage < 2 && !r; stage++) {
       const double t = stage ? tau + ts : tau;
       for (int d = 0; d < (C.bi ? 2 : 3) && !r; d++)
-        r = timed(d, [&]() { return launch_dir<R>(h, P, d, stage, t, d == 0); });
+        r = timed(d, [&]() { return launch_dirs<R>(h, P, d, d + 1, stage, t); });
       if (r) break;
       r = timed(3 + stage, [&]() -> int {
         return stage == 0 ? stage_update<R, 1>(h, P, tau, ts) : stage_update<R, 2>(h, P, tau, ts);
@@ -553,8 +555,12 @@ template <class R>
 static int debug_terms(vh_handle* h, const DevPtrs<R>& P, double* res, double* src, double* du) {
   const DevCfg& C = h->C;
   const long long n = C.n;
-  int r;
-  if ((r = stage_rhs<R>(h, P, 0, h->tau))) return r;
+  // one divergence array: the directions in order, each adding to it (the
+  // staging buffer takes the derivatives below)
+  DevPtrs<R> Q = P;
+  Q.res1 = nullptr;
+  for (int d = 0; d < (C.bi ? 2 : 3); d++)
+    if (int r = launch_dirs<R>(h, Q, d, d + 1, 0, h->tau)) return r;
   R* du16 = reinterpret_cast<R*>(h->stage);
   k_du_full<R><<<grid1(n, 128), 128, 0, h->stream>>>(C, P, du16, h->cfg.dtau);
   // the spatial derivatives along each direction come from k_dir (interior)

@@ -42,10 +42,8 @@ struct Tables {
   int* steps;
   unsigned long long* tmax_bits;
   unsigned int* flag;      // per-event failure bits (the event's DevPtrs status)
-  const int4* xitems;      // {event, tile along x, tile across}
-  int n_x;
-  const int4* yitems;      // {event, tile along y, tile across}
-  int n_y;
+  const int4* items;       // flux tiles: {event, tile along, tile across, cells of a tile + 256 direction}
+  int n_first, n_items;    // tiles up to n_first, then (behind a barrier) the others
   const int2* uitems;      // {event, chunk of blockDim cells}
   int n_u;
   unsigned int* bar;       // [0] arrivals, [1] generation, [2] timeout flag
@@ -98,42 +96,47 @@ __device__ inline bool grid_barrier(unsigned int* bar, long long max_spins = 1ll
   return *(volatile unsigned int*)(bar + 2) == 0;
 }
 
-template <class R, int NC, int MINB, int UNR>
-__global__ void __launch_bounds__(NC * 32, MINB) k_batch(Args<R> A, int nsteps) {
+// one tile of an event's flux sweep along DIR
+template <class R, int DIR>
+__device__ __forceinline__ void event_tile(const DevCfg& C, const DevPtrs<R>& P, int stage, double tau, int4 w,
+                                           R* sm) {
+  const R inv_h = (R)(1.0 / (DIR == 0 ? C.dx : C.dy));
+  if (C.recon == 0)
+    sweep_tile<R, DIR, false, false>(C, P, stage, (R)tau, inv_h, w.w & 255, w.y, w.z, 0, sm);
+  else
+    sweep_tile<R, DIR, true, false>(C, P, stage, (R)tau, inv_h, w.w & 255, w.y, w.z, 0, sm);
+}
+
+template <class R, int MINB>
+__global__ void __launch_bounds__(kSweepThreads, MINB) k_batch(Args<R> A, int nsteps) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  using SX = DirSmem<R, 0, NC>;
-  using SY = DirSmem<R, 1, NC>;
+  R* sm = reinterpret_cast<R*>(smem_raw);
   const Tables& T = A.T;
   __shared__ double red[32];
   for (int s = 0; s < nsteps; s++) {
     for (int stage = 0; stage < 2; stage++) {
-      // ---- flux sweep along x, then y
-      for (int it = blockIdx.x; it < T.n_x; it += gridDim.x) {
-        const int4 w = T.xitems[it];
-        const int ev = w.x;
-        if (T.state[ev] != EV_RUNNING || T.flag[ev]) continue;
-        const DevCfg C = event_cfg(A.C0, T.nx[ev], T.ny[ev]);
-        DevPtrs<R> P = A.pool.shifted(T.off[ev]);
-        P.status = T.flag + ev;
-        const double tau = stage ? T.tau[ev] + T.dtau[ev] : T.tau[ev];
-        dir_tile<R, 0, NC, UNR>(C, P, stage, (R)tau, (R)(1.0 / C.dx), (R)C.dx, 1, w.y, w.z, 0,
-                                *reinterpret_cast<SX*>(smem_raw));
-        __syncthreads();
+      // ---- flux sweeps: all tiles at once where the pool has a divergence
+      // set per direction, else the x tiles and, behind a barrier, the y
+      // tiles that add to them
+      for (int part = 0; part < 2; part++) {
+        const int end = part ? T.n_items : T.n_first;
+        if (part && end == T.n_first) break;
+        for (int it = (part ? T.n_first : 0) + blockIdx.x; it < end; it += gridDim.x) {
+          const int4 w = T.items[it];
+          const int ev = w.x;
+          if (T.state[ev] != EV_RUNNING || T.flag[ev]) continue;
+          const DevCfg C = event_cfg(A.C0, T.nx[ev], T.ny[ev]);
+          DevPtrs<R> P = A.pool.shifted(T.off[ev]);
+          P.status = T.flag + ev;
+          const double tau = stage ? T.tau[ev] + T.dtau[ev] : T.tau[ev];
+          if (w.w >> 8)
+            event_tile<R, 1>(C, P, stage, tau, w, sm);
+          else
+            event_tile<R, 0>(C, P, stage, tau, w, sm);
+          __syncthreads();
+        }
+        if (!grid_barrier(T.bar)) return;
       }
-      if (!grid_barrier(T.bar)) return;
-      for (int it = blockIdx.x; it < T.n_y; it += gridDim.x) {
-        const int4 w = T.yitems[it];
-        const int ev = w.x;
-        if (T.state[ev] != EV_RUNNING || T.flag[ev]) continue;
-        const DevCfg C = event_cfg(A.C0, T.nx[ev], T.ny[ev]);
-        DevPtrs<R> P = A.pool.shifted(T.off[ev]);
-        P.status = T.flag + ev;
-        const double tau = stage ? T.tau[ev] + T.dtau[ev] : T.tau[ev];
-        dir_tile<R, 1, NC, UNR>(C, P, stage, (R)tau, (R)(1.0 / C.dy), (R)C.dy, 0, w.y, w.z, 0,
-                                *reinterpret_cast<SY*>(smem_raw));
-        __syncthreads();
-      }
-      if (!grid_barrier(T.bar)) return;
       // ---- update: sources, RK, root-find, ghosts; stage 2 also reduces max T
       unsigned long long my_it = 0;
       for (int it = blockIdx.x; it < T.n_u; it += gridDim.x) {
@@ -146,8 +149,10 @@ __global__ void __launch_bounds__(NC * 32, MINB) k_batch(Args<R> A, int nsteps) 
         const long long t = (long long)w.y * blockDim.x + threadIdx.x;
         double tg = 0.0;
         if (t < (long long)C.nx * C.ny) {
-          my_it += stage == 0 ? update_cell<R, 1>(C, P, T.tau[ev], T.dtau[ev], t, nullptr)
-                              : update_cell<R, 2>(C, P, T.tau[ev], T.dtau[ev], t, &tg);
+          my_it += stage == 0 ? update_cell<R, 1>(C, P, T.tau[ev], T.dtau[ev], t, nullptr, sm + threadIdx.x,
+                                                     kSweepThreads)
+                              : update_cell<R, 2>(C, P, T.tau[ev], T.dtau[ev], t, &tg, sm + threadIdx.x,
+                                                  kSweepThreads);
         }
         if (stage == 1) {
           for (int o = 16; o > 0; o >>= 1) tg = fmax(tg, __shfl_down_sync(0xffffffffu, tg, o));
@@ -215,12 +220,14 @@ __global__ void k_export_event(DevPtrs<R> P, double* dst, long long n) {
   for (int q = 0; q < 18; q++) dst[q * n + c] = (double)P.f(q)[c];
 }
 
-// one compiled configuration of the persistent kernel
-struct Variant {
-  int nc, minb, unr;
-};
-const Variant kVariants[] = {{4, 4, 1}, {4, 3, 1}, {8, 2, 1}, {8, 2, 3}, {8, 1, 1}};
+// the compiled configurations of the persistent kernel: blocks of 96 threads
+// per SM; more blocks hide more latency, fewer leave more registers.  Measured
+// on 20 events of sides 64..200, 48 steps, tiles of 26 cells (16, 20 and 32:
+// 3 to 7 % slower), in this order: FP32 17.5, 17.0, 16.7, 17.5, 16.6 ms; FP64
+// 26.5, 28.9 and 31.7 ms at 4, 5 and 3 blocks (variants 2 and 3 are 0 and 1).
+constexpr int kBlocks32[] = {8, 7, 5, 6, 4}, kBlocks64[] = {4, 5, 4, 5, 3};
 constexpr int kNumVariants = 5;
+constexpr int kBatchN = 26;  // longest tile, in cells
 const int kStepsChoices[] = {8, 32};
 
 }  // namespace
@@ -244,8 +251,9 @@ struct vh_batch {
   double *d_tau = nullptr, *d_dtau = nullptr, *d_taumax = nullptr;
   unsigned long long *d_tmax = nullptr, *d_iters = nullptr;
   unsigned int *d_flag = nullptr, *d_bar = nullptr;
-  int4 *d_x[2] = {nullptr, nullptr}, *d_y[2] = {nullptr, nullptr};
-  int n_xi[2] = {0, 0}, n_yi[2] = {0, 0};
+  int4* d_items = nullptr;
+  int n_first = 0, n_items = 0;
+  int arrays = 0;  // of the pool: 52, or 61 with a divergence set for y
   int2* d_u = nullptr;
   int n_ui = 0;
   double* stage = nullptr;  // staging for imports (18 x largest event)
@@ -256,6 +264,7 @@ struct vh_batch {
   std::string err;
 };
 
+constexpr int kPoolArrays = 52;
 static std::string g_batch_err;
 
 #define VB_CUDA(b, call)                                                             \
@@ -273,29 +282,28 @@ static DevPtrs<R> pool_ptrs(vh_batch* b) {
   P.base0 = static_cast<R*>(b->pool);
   P.base1 = static_cast<R*>(b->pool) + 18 * b->ntot;
   P.stride = b->ntot;
+  P.res1 = b->arrays > kPoolArrays ? static_cast<R*>(b->pool) + (long long)kPoolArrays * b->ntot : nullptr;
   P.status = nullptr;
   P.iters = b->d_iters;
   return P;
 }
 
 static int build_items(vh_batch* b) {
-  // x and y tiles for NC = 4 and 8 lines, update chunks of the block size
-  for (int q = 0; q < 2; q++) {
-    const int nc = q == 0 ? 4 : 8, tl = 26;
-    std::vector<int4> xs, ys;
-    for (int e = 0; e < b->n; e++) {
-      for (int by = 0; by < (b->ny[e] + nc - 1) / nc; by++)
-        for (int bx = 0; bx < (b->nx[e] + tl - 1) / tl; bx++) xs.push_back(make_int4(e, bx, by, 0));
-      for (int bx = 0; bx < (b->nx[e] + nc - 1) / nc; bx++)
-        for (int by = 0; by < (b->ny[e] + tl - 1) / tl; by++) ys.push_back(make_int4(e, by, bx, 0));
+  // tiles of 8 lines by up to kBatchN cells, an event's tiles of one length
+  std::vector<int4> xs, ys;
+  for (int e = 0; e < b->n; e++) {
+    const int len[2] = {b->nx[e], b->ny[e]};
+    for (int d = 0; d < 2; d++) {
+      const int along = (len[d] + kBatchN - 1) / kBatchN, n = (len[d] + along - 1) / along;
+      for (int by = 0; by < (len[1 - d] + kSweepLines - 1) / kSweepLines; by++)
+        for (int bx = 0; bx < along; bx++) (d ? ys : xs).push_back(make_int4(e, bx, by, n + 256 * d));
     }
-    b->n_xi[q] = (int)xs.size();
-    b->n_yi[q] = (int)ys.size();
-    VB_CUDA(b, cudaMalloc(&b->d_x[q], sizeof(int4) * xs.size()));
-    VB_CUDA(b, cudaMalloc(&b->d_y[q], sizeof(int4) * ys.size()));
-    VB_CUDA(b, cudaMemcpy(b->d_x[q], xs.data(), sizeof(int4) * xs.size(), cudaMemcpyHostToDevice));
-    VB_CUDA(b, cudaMemcpy(b->d_y[q], ys.data(), sizeof(int4) * ys.size(), cudaMemcpyHostToDevice));
   }
+  b->n_first = (int)(b->arrays > kPoolArrays ? xs.size() + ys.size() : xs.size());
+  b->n_items = (int)(xs.size() + ys.size());
+  xs.insert(xs.end(), ys.begin(), ys.end());
+  VB_CUDA(b, cudaMalloc(&b->d_items, sizeof(int4) * xs.size()));
+  VB_CUDA(b, cudaMemcpy(b->d_items, xs.data(), sizeof(int4) * xs.size(), cudaMemcpyHostToDevice));
   return VH_OK;
 }
 
@@ -367,8 +375,16 @@ extern "C" int vh_batch_create(const vh_config* cfg, int n_events, const int* nx
     C.eos_d = b->eos_d; C.eos_f = b->eos_f;
   }
   b->cfg.eos_e = b->cfg.eos_p = b->cfg.eos_cs2 = b->cfg.eos_t = nullptr;
-  const size_t pool_bytes = (size_t)52 * tot * b->esz;
-  cudaError_t ce = cudaMalloc(&b->pool, pool_bytes);
+  // 52 arrays an event, and nine more for the y sweeps' divergence where
+  // they fit
+  b->arrays = kPoolArrays + 9;
+  cudaError_t ce = cudaMalloc(&b->pool, (size_t)b->arrays * tot * b->esz);
+  if (ce == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    b->arrays = kPoolArrays;
+    ce = cudaMalloc(&b->pool, (size_t)b->arrays * tot * b->esz);
+  }
+  const size_t pool_bytes = (size_t)b->arrays * tot * b->esz;
   if (ce != cudaSuccess) { b->err = cudaGetErrorString(ce); g_batch_err = "vh_batch_create: pool: " + b->err; vh_batch_destroy(b); return VH_E_NOMEM; }
   if (!ok(cudaMemset(b->pool, 0, pool_bytes))) return fail("pool");
   const int n = n_events;
@@ -415,7 +431,7 @@ extern "C" int vh_batch_destroy(vh_batch* b) {
   cudaFree(b->d_off); cudaFree(b->d_nx); cudaFree(b->d_ny); cudaFree(b->d_state); cudaFree(b->d_steps);
   cudaFree(b->d_running); cudaFree(b->d_tau); cudaFree(b->d_dtau); cudaFree(b->d_taumax); cudaFree(b->d_tmax);
   cudaFree(b->d_iters); cudaFree(b->d_flag); cudaFree(b->d_bar); cudaFree(b->stage);
-  for (int q = 0; q < 2; q++) { cudaFree(b->d_x[q]); cudaFree(b->d_y[q]); }
+  cudaFree(b->d_items);
   cudaFree(b->d_u);
   delete b;
   return VH_OK;
@@ -493,17 +509,17 @@ extern "C" int vh_batch_init_glauber(vh_batch* b, const uint64_t* seeds, const d
   return VH_OK;
 }
 
-template <class R, int NC, int MINB, int UNR>
+template <class R, int MINB>
 static int launch_variant(vh_batch* b, cudaStream_t s, int nsteps, bool query_only, int* max_blocks) {
-  using SX = DirSmem<R, 0, NC>;
-  using SY = DirSmem<R, 1, NC>;
-  const size_t sm = std::max(sizeof(SX), sizeof(SY));
-  auto kern = k_batch<R, NC, MINB, UNR>;
+  // a sweep's tile, or the update's prefetched values (two divergence sets)
+  const size_t sm = sizeof(R) * std::max({SweepLay<R, 0>(kBatchN).size, SweepLay<R, 1>(kBatchN).size,
+                                          (kPreSlots - 9) * kSweepThreads});
+  auto kern = k_batch<R, MINB>;
   VB_CUDA(b, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   int per_sm = 0, dev = 0, nsm = 0;
   VB_CUDA(b, cudaGetDevice(&dev));
   VB_CUDA(b, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  VB_CUDA(b, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NC * 32, sm));
+  VB_CUDA(b, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSweepThreads, sm));
   const int blocks = std::min(per_sm, MINB) * nsm;
   if (max_blocks) *max_blocks = blocks;
   if (query_only) return blocks > 0 ? VH_OK : VH_E_UNSUPPORTED;
@@ -514,13 +530,12 @@ static int launch_variant(vh_batch* b, cudaStream_t s, int nsteps, bool query_on
   Tables& T = A.T;
   T.n_events = b->n; T.off = b->d_off; T.nx = b->d_nx; T.ny = b->d_ny; T.tau = b->d_tau; T.dtau = b->d_dtau;
   T.tau_max = b->d_taumax; T.state = b->d_state; T.steps = b->d_steps; T.tmax_bits = b->d_tmax; T.flag = b->d_flag;
-  const int q = NC == 4 ? 0 : 1;
-  T.xitems = b->d_x[q]; T.n_x = b->n_xi[q]; T.yitems = b->d_y[q]; T.n_y = b->n_yi[q];
+  T.items = b->d_items; T.n_first = b->n_first; T.n_items = b->n_items;
   T.uitems = b->d_u; T.n_u = b->n_ui; T.bar = b->d_bar; T.running = b->d_running; T.iters = b->d_iters;
   T.t_freeze_gev = b->t_freeze_gev;
   cudaLaunchConfig_t lc{};
   lc.gridDim = dim3(blocks);
-  lc.blockDim = dim3(NC * 32);
+  lc.blockDim = dim3(kSweepThreads);
   lc.dynamicSmemBytes = sm;
   lc.stream = s;
   cudaLaunchAttribute attr[1];
@@ -535,19 +550,19 @@ static int launch_variant(vh_batch* b, cudaStream_t s, int nsteps, bool query_on
 static int launch(vh_batch* b, int variant, cudaStream_t s, int nsteps, bool query_only = false, int* blocks = nullptr) {
   if (b->mixed) {
     switch (variant) {
-      case 0: return launch_variant<float, 4, 4, 1>(b, s, nsteps, query_only, blocks);
-      case 1: return launch_variant<float, 4, 3, 1>(b, s, nsteps, query_only, blocks);
-      case 2: return launch_variant<float, 8, 2, 1>(b, s, nsteps, query_only, blocks);
-      case 3: return launch_variant<float, 8, 2, 3>(b, s, nsteps, query_only, blocks);
-      default: return launch_variant<float, 8, 1, 1>(b, s, nsteps, query_only, blocks);
+      case 0: return launch_variant<float, kBlocks32[0]>(b, s, nsteps, query_only, blocks);
+      case 1: return launch_variant<float, kBlocks32[1]>(b, s, nsteps, query_only, blocks);
+      case 2: return launch_variant<float, kBlocks32[2]>(b, s, nsteps, query_only, blocks);
+      case 3: return launch_variant<float, kBlocks32[3]>(b, s, nsteps, query_only, blocks);
+      default: return launch_variant<float, kBlocks32[4]>(b, s, nsteps, query_only, blocks);
     }
   }
   switch (variant) {
-    case 0: return launch_variant<double, 4, 4, 1>(b, s, nsteps, query_only, blocks);
-    case 1: return launch_variant<double, 4, 3, 1>(b, s, nsteps, query_only, blocks);
-    case 2: return launch_variant<double, 8, 2, 1>(b, s, nsteps, query_only, blocks);
-    case 3: return launch_variant<double, 8, 2, 3>(b, s, nsteps, query_only, blocks);
-    default: return launch_variant<double, 8, 1, 1>(b, s, nsteps, query_only, blocks);
+    case 0: return launch_variant<double, kBlocks64[0]>(b, s, nsteps, query_only, blocks);
+    case 1: return launch_variant<double, kBlocks64[1]>(b, s, nsteps, query_only, blocks);
+    case 2: return launch_variant<double, kBlocks64[2]>(b, s, nsteps, query_only, blocks);
+    case 3: return launch_variant<double, kBlocks64[3]>(b, s, nsteps, query_only, blocks);
+    default: return launch_variant<double, kBlocks64[4]>(b, s, nsteps, query_only, blocks);
   }
 }
 
@@ -558,8 +573,7 @@ static int launch(vh_batch* b, int variant, cudaStream_t s, int nsteps, bool que
 extern "C" int vh_batch_run(vh_batch* b, int max_steps, double* seconds, int* graph_used) {
   if (!b || max_steps < 0) return VH_E_ARG;
   VhNvtxRange range("batched ensemble run");
-  const int block = kVariants[b->variant].nc * 32;
-  if (int r = build_uitems(b, block)) return r;
+  if (int r = build_uitems(b, kSweepThreads)) return r;
   cudaStream_t s;
   VB_CUDA(b, cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
   const int spl = b->steps_per_launch;
@@ -655,9 +669,9 @@ extern "C" int vh_batch_get_tuning(vh_batch* b, int* variant, int* steps_per_lau
   if (!b) return VH_E_ARG;
   if (variant) *variant = b->variant;
   if (steps_per_launch) *steps_per_launch = b->steps_per_launch;
-  if (nc) *nc = kVariants[b->variant].nc;
-  if (minb) *minb = kVariants[b->variant].minb;
-  if (unroll) *unroll = kVariants[b->variant].unr;
+  if (nc) *nc = kSweepLines;
+  if (minb) *minb = (b->mixed ? kBlocks32 : kBlocks64)[b->variant];
+  if (unroll) *unroll = 1;
   return VH_OK;
 }
 
@@ -694,7 +708,7 @@ extern "C" int vh_batch_autotune(vh_batch* b, const char* cache_path, int probe_
     }
   }
   // save the state the trials will advance
-  const size_t pool_bytes = (size_t)52 * b->ntot * b->esz;
+  const size_t pool_bytes = (size_t)b->arrays * b->ntot * b->esz;
   void* save = nullptr;
   VB_CUDA(b, cudaMalloc(&save, pool_bytes));
   // put the saved pool back; on failure free the copy and report

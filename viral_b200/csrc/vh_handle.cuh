@@ -40,9 +40,8 @@ struct vh_handle {
   // the environment at vh_create turns it off, e.g. under a profiler that
   // replays kernels one by one)
   bool pdl = true;
-  // tensor maps of the state for the flux sweeps' TMA tiles, per direction:
-  // [0] arrays 0..4 (e, u^mu), [1] a conserved set (9 arrays)
-  alignas(64) CUtensorMap tmap[3][2];
+  SweepPlan plan{};         // the flux sweeps' tiles
+  TileMaps tmap;            // tensor maps of the state for their TMA staging
   bool tma = false;         // the maps were made (else the sweeps load through the cache)
   bool tma_wanted = true;  // VH_TMA=0 in the environment at vh_create: cached loads
   // discrete-adjoint workspace (kept between calls) and the device
@@ -77,10 +76,12 @@ static inline int fail(vh_handle* h, int code, const std::string& msg) {
 }
 
 template <class R>
-static void set_ptrs(DevPtrs<R>& P, void* base, long long n, unsigned int* status, unsigned long long* iters) {
+static void set_ptrs(DevPtrs<R>& P, void* base, void* res1, long long n, unsigned int* status,
+                     unsigned long long* iters) {
   P.base0 = static_cast<R*>(base);
   P.base1 = static_cast<R*>(base) + 18 * n;
   P.stride = n;
+  P.res1 = static_cast<R*>(res1);
   P.status = status;
   P.iters = iters;
 }
@@ -109,66 +110,39 @@ static cudaError_t launch_step_kernel(bool pdl, K kernel, dim3 grid, dim3 block,
   return cudaLaunchKernelEx(&lc, kernel, args...);
 }
 
+// The flux sweeps of a stage along directions d0..d1-1, one launch.
 template <class R>
-static int launch_dir(vh_handle* h, const DevPtrs<R>& P, int dir, int use_b, double tau, int first) {
+static int launch_dirs(vh_handle* h, const DevPtrs<R>& P, int d0, int d1, int use_b, double tau) {
   const DevCfg& C = h->C;
-  const int nzi = C.kr - C.kl;
-  dim3 grid, block;
-  size_t sm;
-  const double hh = dir == 0 ? C.dx : (dir == 1 ? C.dy : C.dz);
-  const R inv_h = (R)(1.0 / hh), hr = (R)hh;
-  if (dir == 0) {
-    using T = Tile<0, R>;
-    block = dim3(T::NA * T::NC);
-    grid = dim3((C.nx + T::NA - 7) / (T::NA - 6), (C.ny + T::NC - 1) / T::NC, nzi);
-    sm = sizeof(DirSmem<R, 0>);
-    if (h->tma)
-      VH_CUDA(h, launch_step_kernel(h->pdl, k_dir_tma<R, 0>, grid, block, sm, h->stream, C, P, use_b, (R)tau, inv_h,
-                                    hr, first, h->tmap[0][0], h->tmap[0][1]));
-    else
-      VH_CUDA(h, launch_step_kernel(h->pdl, k_dir<R, 0>, grid, block, sm, h->stream, C, P, use_b, (R)tau, inv_h, hr,
-                                    first));
-  } else if (dir == 1) {
-    using T = Tile<1, R>;
-    block = dim3(T::NA * T::NC);
-    grid = dim3((C.ny + T::NA - 7) / (T::NA - 6), (C.ir - C.xt0 + T::NC - 1) / T::NC, nzi);
-    sm = sizeof(DirSmem<R, 1>);
-    if (h->tma)
-      VH_CUDA(h, launch_step_kernel(h->pdl, k_dir_tma<R, 1>, grid, block, sm, h->stream, C, P, use_b, (R)tau, inv_h,
-                                    hr, first, h->tmap[1][0], h->tmap[1][1]));
-    else
-      VH_CUDA(h, launch_step_kernel(h->pdl, k_dir<R, 1>, grid, block, sm, h->stream, C, P, use_b, (R)tau, inv_h, hr,
-                                    first));
-  } else {
-    using T = Tile<2, R>;
-    block = dim3(T::NA * T::NC);
-    grid = dim3((C.nz + T::NA - 7) / (T::NA - 6), (C.ir - C.xt0 + T::NC - 1) / T::NC, C.ny);
-    sm = sizeof(DirSmem<R, 2>);
-    if (h->tma)
-      VH_CUDA(h, launch_step_kernel(h->pdl, k_dir_tma<R, 2>, grid, block, sm, h->stream, C, P, use_b, (R)tau, inv_h,
-                                    hr, first, h->tmap[2][0], h->tmap[2][1]));
-    else
-      VH_CUDA(h, launch_step_kernel(h->pdl, k_dir<R, 2>, grid, block, sm, h->stream, C, P, use_b, (R)tau, inv_h, hr,
-                                    first));
-  }
+  const SweepPlan& p = h->plan;
+  int first = 0, n = 0;
+  for (int d = 0; d < d1; d++) (d < d0 ? first : n) += p.blocks(d);
+  const bool mm = C.recon != 0;
+  // one divergence array for all directions (P.res1 null): the cached kernels
+  auto kern = h->tma && P.res1 ? (mm ? k_dir<R, true, true> : k_dir<R, false, true>)
+                     : (mm ? k_dir<R, true, false> : k_dir<R, false, false>);
+  VH_CUDA(h, launch_step_kernel(h->pdl, kern, dim3(n), dim3(kSweepThreads), sweep_smem<R>(p, C.bi ? 2 : 3), h->stream,
+                                C, P, use_b, (R)tau, p, first, h->tmap));
   return VH_OK;
 }
 
 // The tensor maps of the state: a 4D tensor (x over the padded row pitch,
 // y, z, array) of the 52 arrays, one box shape per sweep direction and
-// array count (TmaBox).  cuTensorMapEncodeTiled comes from the driver
+// array count (SweepLay).  cuTensorMapEncodeTiled comes from the driver
 // through the runtime's entry-point query.
 template <class R, int DIR>
 static int encode_dir_maps(vh_handle* h, PFN_cuTensorMapEncodeTiled_v12000 enc) {
-  using B = TmaBox<R, DIR, Tile<DIR, R>::NC>;
   const DevCfg& C = h->C;
+  const SweepLay<R, DIR> L(h->plan.n[DIR]);
   const cuuint64_t dims[4] = {(cuuint64_t)C.px, (cuuint64_t)C.gy, (cuuint64_t)C.gz, (cuuint64_t)kStateArrays};
   const cuuint64_t strides[3] = {(cuuint64_t)C.px * sizeof(R), (cuuint64_t)C.px * C.gy * sizeof(R),
                                  (cuuint64_t)C.n * sizeof(R)};
   const cuuint32_t estr[4] = {1, 1, 1, 1};
   for (int q = 0; q < 2; q++) {
-    const cuuint32_t box[4] = {(cuuint32_t)B::BX, (cuuint32_t)B::BY, (cuuint32_t)B::BZ, q ? 9u : 5u};
-    const CUresult r = enc(&h->tmap[DIR][q], sizeof(R) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64,
+    const cuuint32_t box[4] = {(cuuint32_t)(DIR == 0 ? L.ld : kSweepLines),
+                               (cuuint32_t)(DIR == 0 ? kSweepLines : DIR == 1 ? L.na : 1),
+                               (cuuint32_t)(DIR == 2 ? L.na : 1), q ? 9u : 5u};
+    const CUresult r = enc(&h->tmap.m[DIR][q], sizeof(R) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64,
                            4, h->state, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -199,23 +173,23 @@ static void encode_maps(vh_handle* h) {
 
 template <class R>
 static int set_smem_attrs(vh_handle* h) {
-  VH_CUDA(h, cudaFuncSetAttribute(k_dir_tma<R, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DirSmem<R, 0>)));
-  VH_CUDA(h, cudaFuncSetAttribute(k_dir_tma<R, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DirSmem<R, 1>)));
-  VH_CUDA(h, cudaFuncSetAttribute(k_dir_tma<R, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DirSmem<R, 2>)));
-  VH_CUDA(h, cudaFuncSetAttribute(k_dir<R, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DirSmem<R, 0>)));
-  VH_CUDA(h, cudaFuncSetAttribute(k_dir<R, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DirSmem<R, 1>)));
-  VH_CUDA(h, cudaFuncSetAttribute(k_dir<R, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DirSmem<R, 2>)));
+  h->plan = sweep_plan<R>(h->C);
   encode_maps<R>(h);
+  VH_CUDA(h, set_sweep_smem(k_dir<R, false, true>));
+  VH_CUDA(h, set_sweep_smem(k_dir<R, true, true>));
+  VH_CUDA(h, set_sweep_smem(k_dir<R, false, false>));
+  VH_CUDA(h, set_sweep_smem(k_dir<R, true, false>));
   return VH_OK;
 }
 
-// the flux-divergence part of a stage: every direction into res, du
+// the flux-divergence part of a stage: every direction into its divergence
+// and du, in one launch
 template <class R>
 static int stage_rhs(vh_handle* h, const DevPtrs<R>& P, int use_b, double tau) {
-  int r;
-  if ((r = launch_dir<R>(h, P, 0, use_b, tau, 1))) return r;
-  if ((r = launch_dir<R>(h, P, 1, use_b, tau, 0))) return r;
-  if (!h->C.bi && (r = launch_dir<R>(h, P, 2, use_b, tau, 0))) return r;
+  const int dirs = h->C.bi ? 2 : 3;
+  if (P.res1) return launch_dirs<R>(h, P, 0, dirs, use_b, tau);
+  for (int d = 0; d < dirs; d++)
+    if (int r = launch_dirs<R>(h, P, d, d + 1, use_b, tau)) return r;
   return VH_OK;
 }
 
@@ -225,7 +199,7 @@ template <class R, int STAGE>
 static int stage_update(vh_handle* h, const DevPtrs<R>& P, double tau, double ts) {
   const DevCfg& C = h->C;
   const long long nint = (long long)C.nx * C.ny * (C.kr - C.kl);
-  VH_CUDA(h, launch_step_kernel(h->pdl, k_update<R, STAGE>, dim3(grid1(nint, 128)), dim3(128), 0, h->stream, C, P,
+  VH_CUDA(h, launch_step_kernel(h->pdl, k_update<R, STAGE>, dim3(grid1(nint, kUpdThreads)), dim3(kUpdThreads), 0, h->stream, C, P,
                                 tau, ts));
   return VH_OK;
 }

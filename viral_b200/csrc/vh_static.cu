@@ -54,12 +54,8 @@ int static_setup(int dev, double** out) {
   if (!g_scratch_ptr[dev]) {
     void* p = nullptr;
     if (cudaGetSymbolAddress(&p, g_vh_static_scratch) != cudaSuccess || !p) return VH_E_CUDA;
-    if (cudaFuncSetAttribute(k_dir<double, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sizeof(DirSmem<double, 0>)) != cudaSuccess ||
-        cudaFuncSetAttribute(k_dir<double, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sizeof(DirSmem<double, 1>)) != cudaSuccess ||
-        cudaFuncSetAttribute(k_dir<double, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sizeof(DirSmem<double, 2>)) != cudaSuccess)
+    if (set_sweep_smem(k_dir<double, false, false>) != cudaSuccess ||
+        set_sweep_smem(k_dir<double, true, false>) != cudaSuccess)
       return VH_E_CUDA;
     g_scratch_ptr[dev] = static_cast<double*>(p);
   }
@@ -112,24 +108,18 @@ int fill_cfg(const vh_config* c, const double* eos_dev, double tau, DevCfg& C) {
   return VH_OK;
 }
 
-int launch_dir_static(const DevCfg& C, const DevPtrs<double>& P, int dir, int use_b, double tau, int first,
-                      cudaStream_t s) {
-  const int nzi = C.kr - C.kl;
-  const double hh = dir == 0 ? C.dx : (dir == 1 ? C.dy : C.dz);
-  if (dir == 0) {
-    using T = Tile<0, double>;
-    dim3 grid((C.nx + T::NA - 7) / (T::NA - 6), (C.ny + T::NC - 1) / T::NC, nzi);
-    k_dir<double, 0><<<grid, dim3(T::NA * T::NC), sizeof(DirSmem<double, 0>), s>>>(C, P, use_b, tau, 1.0 / hh, hh, first);
-  } else if (dir == 1) {
-    using T = Tile<1, double>;
-    dim3 grid((C.ny + T::NA - 7) / (T::NA - 6), (C.ir - C.xt0 + T::NC - 1) / T::NC, nzi);
-    k_dir<double, 1><<<grid, dim3(T::NA * T::NC), sizeof(DirSmem<double, 1>), s>>>(C, P, use_b, tau, 1.0 / hh, hh, first);
-  } else {
-    using T = Tile<2, double>;
-    dim3 grid((C.nz + T::NA - 7) / (T::NA - 6), (C.ir - C.xt0 + T::NC - 1) / T::NC, C.ny);
-    k_dir<double, 2><<<grid, dim3(T::NA * T::NC), sizeof(DirSmem<double, 2>), s>>>(C, P, use_b, tau, 1.0 / hh, hh, first);
+// The sweeps of a stage one direction after the other, each adding to the one
+// divergence array the scratch has room for.
+int launch_dirs_static(const DevCfg& C, const DevPtrs<double>& P, const SweepPlan& plan, int use_b, double tau,
+                       cudaStream_t s) {
+  const TileMaps none{};  // read by the TMA-staged kernels alone
+  const int dirs = C.bi ? 2 : 3;
+  for (int d = 0, first = 0; d < dirs; first += plan.blocks(d++)) {
+    auto kern = C.recon != 0 ? k_dir<double, true, false> : k_dir<double, false, false>;
+    kern<<<plan.blocks(d), kSweepThreads, sweep_smem<double>(plan, dirs), s>>>(C, P, use_b, tau, plan, first, none);
+    if (cudaGetLastError() != cudaSuccess) return VH_E_CUDA;
   }
-  return cudaGetLastError() == cudaSuccess ? VH_OK : VH_E_CUDA;
+  return VH_OK;
 }
 
 }  // namespace
@@ -155,16 +145,16 @@ extern "C" int vh_step_static(const vh_config* cfg, double* state, const double*
   P.iters = reinterpret_cast<unsigned long long*>(scratch + 1);
   if (cudaMemsetAsync(scratch, 0, kHeaderDoubles * sizeof(double), s) != cudaSuccess) return VH_E_CUDA;
 
+  const SweepPlan plan = sweep_plan<double>(C);
   const double ts = cfg->dtau;
   const long long nint = (long long)C.nx * C.ny * (C.kr - C.kl);
-  const unsigned blocks = (unsigned)((nint + 127) / 128);
+  const unsigned blocks = (unsigned)((nint + kUpdThreads - 1) / kUpdThreads);
   for (int st = 0; st < nsteps; st++) {
     for (int stage = 0; stage < 2; stage++) {
       const double t = stage ? tau + ts : tau;
-      for (int d = 0; d < (C.bi ? 2 : 3); d++)
-        if (int r = launch_dir_static(C, P, d, stage, t, d == 0, s)) return r;
-      if (stage == 0) k_update<double, 1><<<blocks, 128, 0, s>>>(C, P, tau, ts);
-      else k_update<double, 2><<<blocks, 128, 0, s>>>(C, P, tau, ts);
+      if (int r = launch_dirs_static(C, P, plan, stage, t, s)) return r;
+      if (stage == 0) k_update<double, 1><<<blocks, kUpdThreads, 0, s>>>(C, P, tau, ts);
+      else k_update<double, 2><<<blocks, kUpdThreads, 0, s>>>(C, P, tau, ts);
       if (cudaGetLastError() != cudaSuccess) return VH_E_CUDA;
     }
     tau += ts;
