@@ -140,3 +140,30 @@ def test_freezeout_step_follows_a_run():
         assert A.lib().vh_freezeout_step(H.h, tfo, small.data_ptr(), 2, ctypes.byref(cnt)) == A.E_ARG
         assert cnt.value == len(want)
         same_elements(H.freezeout_step(tfo), want)
+
+
+@pytest.mark.parametrize("count", [0, 1, 127, 129, 700])
+@pytest.mark.parametrize("npt,nphi", [(1, 1), (3, 15), (2, 16), (3, 17), (1, 33), (1030, 1), (2, 8200)])
+def test_spectrum_bin_tiles(npt, nphi, count):
+    """bins around the tile of 16 and the launch of 1024 tiles, elements
+    around a block's 128, against the host sum; every term is positive, so
+    the sums agree to the rounding of the exponents (below 100, 1e-14 each
+    side) and of the terms' products"""
+    rng = np.random.default_rng(npt + nphi + count)
+    if npt * nphi > 1000 and count > 1:
+        count = 3 if count < 200 else 130
+    pt, phi = np.linspace(0.1, 2.0, npt), np.linspace(0, 2 * np.pi, nphi, endpoint=False)
+    v = 0.3 * rng.standard_normal((3, count))
+    for width, dev_fn, host_fn, rap in ((9, cooper_frye_2d_device, cooper_frye_2d, ()),
+                                        (12, cooper_frye_3d_device, cooper_frye_3d, (0.3,))):
+        w = width // 3
+        el = np.zeros((count, width))
+        el[:, 0] = 1 + rng.random(count)
+        el[:, 1:w] = rng.standard_normal((count, w - 1)) * 0.5
+        el[:, w] = 1 + rng.random(count)
+        el[:, w + 1:2 * w] = 0.1 * rng.standard_normal((count, w - 1))
+        el[:, 2 * w + 1:] = v[:w - 1].T
+        el[:, 2 * w] = np.sqrt(1 + (v[:2] ** 2).sum(0) + (el[:, 0] * v[2]) ** 2 * (w == 4))
+        host = host_fn(el, 0.15, 0.7, 3.0, *rap, pt, phi)
+        got = dev_fn(dev(el), 0.15, 0.7, 3.0, *rap, pt, phi)
+        assert np.allclose(got, host, rtol=1e-12, atol=0)

@@ -91,8 +91,10 @@ VH_FO_HD void kuhn_simplex(int s, int m, int* v) {
 // 2 y, 3 eta); lo, hi: the two coordinates per axis; f = T - T_fo
 template <int D>
 struct Corners {
-  double lo[D], hi[D], u[1 << D][D], f[1 << D];
+  double lo[D], hi[D], uv[1 << D][D], fv[1 << D];
   VH_FO_HD double x(int v, int q) const { return ((v >> q) & 1) ? hi[q] : lo[q]; }
+  VH_FO_HD double f(int v) const { return fv[v]; }
+  VH_FO_HD double u(int v, int q) const { return uv[v][q]; }
 };
 
 // cell index of corner v of cube (i, j, k) in its time slice
@@ -109,8 +111,8 @@ VH_FO_HD bool load(const Geo& g, int i, int j, int k, const double* t0, const do
                    const double* u1, Corners<D>& K) {
   bool pos = false, neg = false;
   for (int v = 0; v < (1 << D); v++) {
-    K.f[v] = ((v & 1) ? t1 : t0)[corner_cell<D>(g, i, j, k, v)] - g.t_fo;
-    if (K.f[v] > 0) pos = true; else neg = true;
+    K.fv[v] = ((v & 1) ? t1 : t0)[corner_cell<D>(g, i, j, k, v)] - g.t_fo;
+    if (K.fv[v] > 0) pos = true; else neg = true;
   }
   if (!pos || !neg) return false;
   K.lo[0] = g.tau0;
@@ -126,7 +128,7 @@ VH_FO_HD bool load(const Geo& g, int i, int j, int k, const double* t0, const do
   for (int v = 0; v < (1 << D); v++) {
     const long long c = corner_cell<D>(g, i, j, k, v);
     const double* U = (v & 1) ? u1 : u0;
-    for (int q = 0; q < D; q++) K.u[v][q] = U[q * g.n + c];
+    for (int q = 0; q < D; q++) K.uv[v][q] = U[q * g.n + c];
   }
   return true;
 }
@@ -157,14 +159,14 @@ template <int D>
 struct Pt {
   double x[D], u[D];
 };
-template <int D>
-VH_FO_HD Pt<D> edge_point(const Corners<D>& K, int a, int b) {
-  const double w = K.f[a] / (K.f[a] - K.f[b]);
+template <int D, class K_>
+VH_FO_HD Pt<D> edge_point(const K_& K, int a, int b) {
+  const double w = K.f(a) / (K.f(a) - K.f(b));
   Pt<D> p;
   for (int q = 0; q < D; q++) {
     const double xa = K.x(a, q), xb = K.x(b, q);
     p.x[q] = xa + w * (xb - xa);
-    p.u[q] = K.u[a][q] + w * (K.u[b][q] - K.u[a][q]);
+    p.u[q] = K.u(a, q) + w * (K.u(b, q) - K.u(a, q));
   }
   return p;
 }
@@ -228,34 +230,75 @@ VH_FO_HD void tetra(const Pt<4>& a, const Pt<4>& b, const Pt<4>& c, const Pt<4>&
   s.put(o, kW3);
 }
 
+// every element of one simplex of a cube, v its vertices: a tetrahedron of
+// the (tau, x, y) cube gives 0, 1 or 2 triangles.  K: the cube's corners
+// (f, x, u of corner v), on the host all loaded, on the device read as needed.
+template <class K3>
+VH_FO_HD void simplex2(const K3& K, const int* v, Sink& s) {
+  int hot[4], cold[4], nh = 0, nc = 0;
+  for (int q = 0; q < 4; q++) {
+    if (K.f(v[q]) > 0) hot[nh++] = v[q]; else cold[nc++] = v[q];
+  }
+  if (!nh || !nc) return;
+  double ph[3], pc[3];  // a hot and a cold corner: the orientation
+  for (int q = 0; q < 3; q++) {
+    ph[q] = K.x(hot[0], q);
+    pc[q] = K.x(cold[0], q);
+  }
+  if (nh == 1 || nc == 1) {
+    const int lone = nh == 1 ? hot[0] : cold[0];
+    const int* o = nh == 1 ? cold : hot;
+    triangle(edge_point<3>(K, lone, o[0]), edge_point<3>(K, lone, o[1]), edge_point<3>(K, lone, o[2]), pc, ph, s);
+  } else {
+    // two against two: the quadrilateral a-b-c-d as two triangles
+    const Pt<3> a = edge_point<3>(K, hot[0], cold[0]), b = edge_point<3>(K, hot[0], cold[1]);
+    const Pt<3> c = edge_point<3>(K, hot[1], cold[1]), d = edge_point<3>(K, hot[1], cold[0]);
+    triangle(a, b, c, pc, ph, s);
+    triangle(a, c, d, pc, ph, s);
+  }
+}
+
+// a 4-simplex of the (tau, x, y, eta) hypercube: 0, 1 or 3 tetrahedra
+template <class K4>
+VH_FO_HD void simplex3(const K4& K, const int* v, Sink& s) {
+  int hot[5], cold[5], nh = 0, nc = 0;
+  for (int q = 0; q < 5; q++) {
+    if (K.f(v[q]) > 0) hot[nh++] = v[q]; else cold[nc++] = v[q];
+  }
+  if (!nh || !nc) return;
+  double ph[4], pc[4];  // a hot and a cold corner: the orientation
+  for (int q = 0; q < 4; q++) {
+    ph[q] = K.x(hot[0], q);
+    pc[q] = K.x(cold[0], q);
+  }
+  if (nh == 1 || nc == 1) {
+    // one vertex against four: a tetrahedron
+    const int lone = nh == 1 ? hot[0] : cold[0];
+    const int* o = nh == 1 ? cold : hot;
+    tetra(edge_point<4>(K, lone, o[0]), edge_point<4>(K, lone, o[1]), edge_point<4>(K, lone, o[2]),
+          edge_point<4>(K, lone, o[3]), pc, ph, s);
+  } else {
+    // two against three: a triangular prism, as three tetrahedra
+    const int* two = nh == 2 ? hot : cold;
+    const int* three = nh == 2 ? cold : hot;
+    const Pt<4> a0 = edge_point<4>(K, two[0], three[0]), a1 = edge_point<4>(K, two[0], three[1]);
+    const Pt<4> a2 = edge_point<4>(K, two[0], three[2]), b0 = edge_point<4>(K, two[1], three[0]);
+    const Pt<4> b1 = edge_point<4>(K, two[1], three[1]), b2 = edge_point<4>(K, two[1], three[2]);
+    tetra(a0, a1, a2, b0, pc, ph, s);
+    tetra(a1, a2, b0, b1, pc, ph, s);
+    tetra(a2, b0, b1, b2, pc, ph, s);
+  }
+}
+
 // every element of cube (i, j, k) in 2+1D (k unused): marching tetrahedra
 VH_FO_HD void cube2(const Geo& g, int i, int j, const double* t0, const double* t1, const double* u0,
                     const double* u1, Sink& s) {
   Corners<3> K;
   if (!load<3>(g, i, j, kG, t0, t1, u0, u1, K)) return;
   for (int sx = 0; sx < 6; sx++) {
-    int v[4], hot[4], cold[4], nh = 0, nc = 0;
+    int v[4];
     kuhn_simplex(sx, 3, v);
-    for (int q = 0; q < 4; q++) {
-      if (K.f[v[q]] > 0) hot[nh++] = v[q]; else cold[nc++] = v[q];
-    }
-    if (!nh || !nc) continue;
-    double ph[3], pc[3];  // a hot and a cold corner: the orientation
-    for (int q = 0; q < 3; q++) {
-      ph[q] = K.x(hot[0], q);
-      pc[q] = K.x(cold[0], q);
-    }
-    if (nh == 1 || nc == 1) {
-      const int lone = nh == 1 ? hot[0] : cold[0];
-      const int* o = nh == 1 ? cold : hot;
-      triangle(edge_point(K, lone, o[0]), edge_point(K, lone, o[1]), edge_point(K, lone, o[2]), pc, ph, s);
-    } else {
-      // two against two: the quadrilateral a-b-c-d as two triangles
-      const Pt<3> a = edge_point(K, hot[0], cold[0]), b = edge_point(K, hot[0], cold[1]);
-      const Pt<3> c = edge_point(K, hot[1], cold[1]), d = edge_point(K, hot[1], cold[0]);
-      triangle(a, b, c, pc, ph, s);
-      triangle(a, c, d, pc, ph, s);
-    }
+    simplex2(K, v, s);
   }
 }
 
@@ -265,34 +308,9 @@ VH_FO_HD void cube3(const Geo& g, int i, int j, int k, const double* t0, const d
   Corners<4> K;
   if (!load<4>(g, i, j, k, t0, t1, u0, u1, K)) return;
   for (int sx = 0; sx < 24; sx++) {
-    int v[5], hot[5], cold[5], nh = 0, nc = 0;
+    int v[5];
     kuhn_simplex(sx, 4, v);
-    for (int q = 0; q < 5; q++) {
-      if (K.f[v[q]] > 0) hot[nh++] = v[q]; else cold[nc++] = v[q];
-    }
-    if (!nh || !nc) continue;
-    double ph[4], pc[4];  // a hot and a cold corner: the orientation
-    for (int q = 0; q < 4; q++) {
-      ph[q] = K.x(hot[0], q);
-      pc[q] = K.x(cold[0], q);
-    }
-    if (nh == 1 || nc == 1) {
-      // one vertex against four: a tetrahedron
-      const int lone = nh == 1 ? hot[0] : cold[0];
-      const int* o = nh == 1 ? cold : hot;
-      tetra(edge_point(K, lone, o[0]), edge_point(K, lone, o[1]), edge_point(K, lone, o[2]),
-            edge_point(K, lone, o[3]), pc, ph, s);
-    } else {
-      // two against three: a triangular prism, as three tetrahedra
-      const int* two = nh == 2 ? hot : cold;
-      const int* three = nh == 2 ? cold : hot;
-      const Pt<4> a0 = edge_point(K, two[0], three[0]), a1 = edge_point(K, two[0], three[1]);
-      const Pt<4> a2 = edge_point(K, two[0], three[2]), b0 = edge_point(K, two[1], three[0]);
-      const Pt<4> b1 = edge_point(K, two[1], three[1]), b2 = edge_point(K, two[1], three[2]);
-      tetra(a0, a1, a2, b0, pc, ph, s);
-      tetra(a1, a2, b0, b1, pc, ph, s);
-      tetra(a2, b0, b1, b2, pc, ph, s);
-    }
+    simplex3(K, v, s);
   }
 }
 

@@ -1,11 +1,12 @@
 // Isothermal freeze-out hypersurface and Cooper-Frye spectra on the GPU,
-// from device arrays: the per-cube arithmetic of vh_freezeout.cuh, one
-// thread per space-time cube, in two passes so that the elements land in the
-// host entry points' order (cube order, x fastest) without atomics: a count
-// pass from the signs of T - T_fo alone, an exclusive scan of the counts, and
-// an emit pass in which each cut cube writes its elements from its offset.
-// The spectra are a reduction over the elements per momentum bin, one block
-// per bin with a fixed summation tree (deterministic).
+// from device arrays: the per-simplex arithmetic of vh_freezeout.cuh, in two
+// passes so that the elements land in the host entry points' order (cube
+// order, x fastest): a count pass from the signs of T - T_fo alone, which also
+// lists the cut cubes, an exclusive scan of the counts, and an emit pass, a
+// group of lanes per cut cube and a lane per simplex, that writes the cube's
+// elements from its offset.  The list's order varies from run to run, the
+// elements' places do not.  The spectra are sums over the elements per
+// momentum bin in a fixed order (deterministic).
 #include <cuda_runtime.h>
 
 #include <climits>
@@ -22,55 +23,179 @@ namespace {
 
 constexpr int kThreads = 256;
 
+// counts[c]: elements of cube c; list[0 .. *ncut): the cubes with any
 template <int D>
 __global__ void __launch_bounds__(kThreads) k_fo_count(vh_fo::Geo g, const double* __restrict__ t0,
                                                         const double* __restrict__ t1, long long ncubes,
-                                                        long long* __restrict__ counts) {
+                                                        long long* __restrict__ counts, int* __restrict__ list,
+                                                        int* __restrict__ ncut) {
   const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ncubes) return;
-  int i, j, k;
-  vh_fo::cube_ijk(g, c, &i, &j, &k);
-  counts[c] = vh_fo::count<D>(g, i, j, k, t0, t1);
+  long long n = 0;
+  if (c < ncubes) {
+    int i, j, k;
+    vh_fo::cube_ijk(g, c, &i, &j, &k);
+    counts[c] = n = vh_fo::count<D>(g, i, j, k, t0, t1);
+  }
+  const unsigned cut = __ballot_sync(0xffffffffu, n != 0);
+  if (cut == 0) return;
+  const int lane = threadIdx.x & 31;
+  int at = 0;
+  if (lane == 0) at = atomicAdd(ncut, __popc(cut));
+  at = __shfl_sync(0xffffffffu, at, 0);
+  if (n) list[at + __popc(cut & ((1u << lane) - 1))] = (int)c;
 }
 
+// a cube's corners, read where a simplex needs them
+template <int D>
+struct CornersAt {
+  const vh_fo::Geo& g;
+  const double *t0, *t1, *u0, *u1;
+  int i, j, k;
+  double lo[D], hi[D];
+  __device__ __forceinline__ double x(int v, int q) const { return ((v >> q) & 1) ? hi[q] : lo[q]; }
+  __device__ __forceinline__ double f(int v) const {
+    return ((v & 1) ? t1 : t0)[vh_fo::corner_cell<D>(g, i, j, k, v)] - g.t_fo;
+  }
+  __device__ __forceinline__ double u(int v, int q) const {
+    return ((v & 1) ? u1 : u0)[q * g.n + vh_fo::corner_cell<D>(g, i, j, k, v)];
+  }
+};
+
+// A cut cube takes a whole warp in 3+1D (24 simplices) and 8 lanes in 2+1D
+// (6).  A thread per cube had left one or two lanes of a warp at work, each
+// on 24 simplices in turn from its own stack (121x121x31, 0.8 M elements:
+// 0.92 ms; now 0.15).
 template <int D>
 __global__ void __launch_bounds__(kThreads) k_fo_emit(vh_fo::Geo g, const double* __restrict__ t0,
                                                        const double* __restrict__ t1, const double* __restrict__ u0,
-                                                       const double* __restrict__ u1, long long ncubes,
-                                                       const long long* __restrict__ counts,
+                                                       const double* __restrict__ u1, const int* __restrict__ list,
+                                                       const int* __restrict__ ncut,
                                                        const long long* __restrict__ offs, double* __restrict__ out,
                                                        long long cap) {
-  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ncubes || counts[c] == 0) return;
-  int i, j, k;
-  vh_fo::cube_ijk(g, c, &i, &j, &k);
-  vh_fo::Sink s{out, offs[c], cap};  // writes below cap only
-  if (D == 3)
-    vh_fo::cube2(g, i, j, t0, t1, u0, u1, s);
-  else
-    vh_fo::cube3(g, i, j, k, t0, t1, u0, u1, s);
+  constexpr int G = D == 3 ? 8 : 32, S = D == 3 ? 6 : 24, MANY = D == 3 ? 2 : 3;
+  const int lane = threadIdx.x & 31, sx = lane % G, first = lane - sx;
+  int v[5];
+  vh_fo::kuhn_simplex(sx < S ? sx : 0, D, v);
+  const int n = *ncut;
+  const long long groups = (long long)gridDim.x * (kThreads / G);
+  for (long long at = (long long)blockIdx.x * (kThreads / G) + threadIdx.x / G;; at += groups) {
+    // the warp's groups step together: their lanes meet in the ballots
+    if (!__any_sync(0xffffffffu, at < n)) break;
+    const bool live = at < n && sx < S;
+    const long long c = at < n ? list[at] : 0;
+    CornersAt<D> K{g, t0, t1, u0, u1, 0, 0, 0, {}, {}};
+    vh_fo::cube_ijk(g, c, &K.i, &K.j, &K.k);
+    K.lo[0] = g.tau0;
+    K.hi[0] = g.tau1;
+    K.lo[1] = g.x0 + (K.i - vh_fo::kG) * g.dx;
+    K.hi[1] = g.x0 + (K.i + 1 - vh_fo::kG) * g.dx;
+    K.lo[2] = g.y0 + (K.j - vh_fo::kG) * g.dy;
+    K.hi[2] = g.y0 + (K.j + 1 - vh_fo::kG) * g.dy;
+    if (D == 4) {
+      K.lo[D - 1] = g.z0 + (K.k - vh_fo::kG) * g.dz;
+      K.hi[D - 1] = g.z0 + (K.k + 1 - vh_fo::kG) * g.dz;
+    }
+    int nh = 0;
+    if (live)
+      for (int q = 0; q <= D; q++) nh += K.f(v[q]) > 0;
+    const int nc = D + 1 - nh;
+    const bool cut = live && nh && nc, lone = cut && (nh == 1 || nc == 1);
+    // the elements of the cube's simplices before this one
+    const unsigned before = ((1u << lane) - 1) & ~((1u << first) - 1);
+    const unsigned one = __ballot_sync(0xffffffffu, lone) & before, many = __ballot_sync(0xffffffffu, cut && !lone) & before;
+    if (cut) {
+      vh_fo::Sink s{out, offs[c] + __popc(one) + MANY * __popc(many), cap};  // writes below cap only
+      if constexpr (D == 3)
+        vh_fo::simplex2(K, v, s);
+      else
+        vh_fo::simplex3(K, v, s);
+    }
+  }
 }
 
-// one block per momentum bin (m_T, p_x, p_y); the block's threads stride
-// over the elements and add their partial sums in a fixed tree
+// ---- spectra
+// A block sums a share of the elements for kBins momentum bins at once, one
+// element a thread at a time: what depends on the element alone (in 3+1D
+// cosh and sinh of y - eta; in 2+1D the Bessel functions, which depend on the
+// bin through m_T only) is formed once for all of them, and the bins'
+// exponentials are independent of one another.  One block per bin had formed
+// them per bin, with 128 blocks on the GPU (0.8 M elements, 8 x 16 bins:
+// 4.06 ms; now 0.78, bound by the FP64 exponentials).  bins: m_T, p_x, p_y, kBins a tile, zeros where a tile has fewer;
+// part: a partial sum per bin and share of the elements.
+constexpr int kBins = 16, kCfThreads = 128;
 template <int D>
-__global__ void __launch_bounds__(kThreads) k_cooper_frye(const double* __restrict__ el, long long count,
-                                                           const double* __restrict__ bins, double y, double t_fo,
-                                                           double pref, double* __restrict__ out) {
-  __shared__ double red[kThreads];
-  const long long b = blockIdx.x;
-  const double mt = bins[3 * b], px = bins[3 * b + 1], py = bins[3 * b + 2];
-  double s = 0;
-  for (long long e = threadIdx.x; e < count; e += kThreads)
-    s += D == 3 ? vh_fo::cf2_term(el + vh_fo::kW2 * e, mt, px, py, t_fo)
-                : vh_fo::cf3_term(el + vh_fo::kW3 * e, mt, px, py, y, t_fo);
-  red[threadIdx.x] = s;
+__global__ void __launch_bounds__(kCfThreads, 4) k_cooper_frye(const double* __restrict__ el, long long count,
+                                                             const double* __restrict__ bins, double y, double t_fo,
+                                                             double* __restrict__ part) {
+  __shared__ double bin[kBins][3], red[kCfThreads / 32][kBins];
+  const int tid = threadIdx.x;
+  if (tid < 3 * kBins) bin[tid / 3][tid % 3] = bins[(long long)blockIdx.x * 3 * kBins + tid];
   __syncthreads();
-  for (int w = kThreads / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-    __syncthreads();
+  const double it = 1.0 / t_fo;
+  double acc[kBins];
+#pragma unroll
+  for (int b = 0; b < kBins; b++) acc[b] = 0;
+  for (long long e = (long long)blockIdx.y * kCfThreads + tid; e < count; e += (long long)gridDim.y * kCfThreads) {
+    if constexpr (D == 4) {
+      const double* q = el + vh_fo::kW3 * e;
+      const double tau = q[0], ch = cosh(y - q[3]), sh = sinh(y - q[3]);
+      // p.dSigma = m_T A + p_x B + p_y C, p.u / T = m_T U - p_x V - p_y W
+      const double A = ch * q[4] + sh / tau * q[7], B = q[5], C = q[6];
+      const double U = (ch * q[8] - tau * sh * q[11]) * it, V = q[9] * it, W = q[10] * it;
+#pragma unroll
+      for (int b = 0; b < kBins; b++) {
+        const double mt = bin[b][0], px = bin[b][1], py = bin[b][2];
+        acc[b] += (mt * A + px * B + py * C) * exp(px * V + py * W - mt * U);
+      }
+    } else {
+      const double* q = el + vh_fo::kW2 * e;
+      const double mt = bin[0][0], a = mt * q[6] * it;
+      double k0e, k1e;
+      vh_fo::bessel_k01e(a, &k0e, &k1e);
+      const double A = 2 * mt * k1e * q[3], B = 2 * k0e * q[4], C = 2 * k0e * q[5], V = q[7] * it, W = q[8] * it;
+#pragma unroll
+      for (int b = 0; b < kBins; b++) {
+        const double px = bin[b][1], py = bin[b][2];
+        acc[b] += (A + px * B + py * C) * exp(px * V + py * W - a);
+      }
+    }
   }
-  if (threadIdx.x == 0) out[b] = pref * red[0];
+#pragma unroll
+  for (int b = 0; b < kBins; b++) {
+    for (int o = 16; o > 0; o >>= 1) acc[b] += __shfl_down_sync(0xffffffffu, acc[b], o);
+    if ((tid & 31) == 0) red[tid >> 5][b] = acc[b];
+  }
+  __syncthreads();
+  if (tid < kBins) {
+    double s = 0;
+    for (int w = 0; w < kCfThreads / 32; w++) s += red[w][tid];
+    part[((long long)blockIdx.x * kBins + tid) * gridDim.y + blockIdx.y] = s;
+  }
+}
+// the shares' sums, one warp per slot; slot q of tile t is the bin
+// first_bin(t) + q of the spectrum
+struct CfTiles {
+  int nphi, per_row;  // per_row: tiles of a p_T (2+1D), 0: tiles run on over the bins (3+1D)
+  long long nb;
+  __host__ __device__ long long first(long long t) const {
+    return per_row ? t / per_row * nphi + t % per_row * kBins : t * kBins;
+  }
+  __host__ __device__ long long end(long long t) const {
+    const long long f = first(t) + kBins, m = per_row ? (t / per_row + 1) * nphi : nb;
+    return f < m ? f : m;
+  }
+};
+__global__ void k_cf_final(const double* __restrict__ part, int shares, CfTiles tl, long long tile0, int tiles,
+                           double pref, double* __restrict__ out) {
+  const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / 32;
+  const int lane = threadIdx.x & 31;
+  if (w >= (long long)tiles * kBins) return;
+  const long long t = tile0 + w / kBins, bin = tl.first(t) + w % kBins;
+  if (bin >= tl.end(t)) return;
+  double s = 0;
+  for (int k = lane; k < shares; k += 32) s += part[w * shares + k];
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if (lane == 0) out[bin] = pref * s;
 }
 
 inline unsigned blocks(long long n) { return (unsigned)((n + kThreads - 1) / kThreads); }
@@ -88,8 +213,10 @@ int surface(const vh_fo::Geo& g, const double* t0, const double* t1, const doubl
   if (cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, scan_in, scan_out, (int)nc, st) != cudaSuccess)
     return VH_E_CUDA;
   const size_t words = 2 * (size_t)nc;  // counts, offsets
+  const size_t ints = (size_t)nc + 1;   // cut cubes and their number
   char* buf = nullptr;
-  if (cudaMallocAsync((void**)&buf, words * sizeof(long long) + scan_bytes + 256, st) != cudaSuccess) {
+  if (cudaMallocAsync((void**)&buf, words * sizeof(long long) + ints * sizeof(int) + scan_bytes + 512, st) !=
+      cudaSuccess) {
     cudaGetLastError();
     return VH_E_NOMEM;
   }
@@ -97,17 +224,22 @@ int surface(const vh_fo::Geo& g, const double* t0, const double* t1, const doubl
   long long* offs = counts + nc;
   scan_in = counts;
   scan_out = offs;
-  void* scan_tmp = buf + ((words * sizeof(long long) + 255) / 256) * 256;
+  int* list = reinterpret_cast<int*>(offs + nc);
+  int* ncut = list + nc;
+  void* scan_tmp = buf + ((words * sizeof(long long) + ints * sizeof(int) + 255) / 256) * 256;
   int rc = VH_OK;
   long long tail[2] = {0, 0};
-  k_fo_count<D><<<blocks(nc), kThreads, 0, st>>>(g, t0, t1, nc, counts);
+  if (cudaMemsetAsync(ncut, 0, sizeof(int), st) != cudaSuccess) rc = VH_E_CUDA;
+  k_fo_count<D><<<blocks(nc), kThreads, 0, st>>>(g, t0, t1, nc, counts, list, ncut);
   if (cudaGetLastError() != cudaSuccess ||
       cub::DeviceScan::ExclusiveSum(scan_tmp, scan_bytes, scan_in, scan_out, (int)nc, st) != cudaSuccess ||
       cudaMemcpyAsync(&tail[0], offs + nc - 1, sizeof(long long), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
       cudaMemcpyAsync(&tail[1], counts + nc - 1, sizeof(long long), cudaMemcpyDeviceToHost, st) != cudaSuccess)
     rc = VH_E_CUDA;
   if (rc == VH_OK && cap > 0) {
-    k_fo_emit<D><<<blocks(nc), kThreads, 0, st>>>(g, t0, t1, u0, u1, nc, counts, offs, out, cap);
+    // as many warps as an SM holds, each taking cut cubes in turn
+    const unsigned most = 148 * 8, need = blocks(nc * (D == 3 ? 8 : 32));
+    k_fo_emit<D><<<need < most ? need : most, kThreads, 0, st>>>(g, t0, t1, u0, u1, list, ncut, offs, out, cap);
     if (cudaGetLastError() != cudaSuccess) rc = VH_E_CUDA;
   }
   if (cudaFreeAsync(buf, st) != cudaSuccess && rc == VH_OK) rc = VH_E_CUDA;
@@ -124,30 +256,51 @@ int spectrum(const double* el, long long count, double t_fo, double mass, double
   const long long nb = (long long)npt * nphi;
   if (nb > INT_MAX) return VH_E_ARG;
   VhNvtxRange range("Cooper-Frye spectrum");
-  std::vector<double> bins(3 * (size_t)nb);
-  for (int a = 0; a < npt; a++)
-    for (int b = 0; b < nphi; b++) {
-      double* q = &bins[3 * ((size_t)a * nphi + b)];
-      q[0] = std::sqrt(mass * mass + pt[a] * pt[a]);
-      q[1] = pt[a] * std::cos(phi[b]);
-      q[2] = pt[a] * std::sin(phi[b]);
+  // bins in tiles of kBins: in 2+1D the azimuths of one p_T (the Bessel
+  // functions depend on p_T alone), in 3+1D any; kMostTiles tiles a launch,
+  // which bounds the scratch
+  constexpr long long kMostTiles = 1024;
+  const CfTiles tl{nphi, D == 3 ? (nphi + kBins - 1) / kBins : 0, nb};
+  const long long tiles = D == 3 ? (long long)npt * tl.per_row : (nb + kBins - 1) / kBins;
+  const int chunk = (int)(tiles < kMostTiles ? tiles : kMostTiles);
+  // shares of the elements: about four blocks per SM over the tiles
+  const long long most = (count + kCfThreads - 1) / kCfThreads;
+  long long shares = (4 * 148 + chunk - 1) / chunk;
+  shares = shares > most ? most : shares;
+  shares = shares < 1 ? 1 : shares;
+  std::vector<double> bins(3 * kBins * (size_t)tiles, 0.0);
+  for (long long t = 0; t < tiles; t++)
+    for (long long i = tl.first(t); i < tl.end(t); i++) {
+      double* q = &bins[3 * (size_t)(t * kBins + i - tl.first(t))];
+      const double p = pt[i / nphi], f = phi[i % nphi];
+      q[0] = std::sqrt(mass * mass + p * p);
+      q[1] = p * std::cos(f);
+      q[2] = p * std::sin(f);
     }
+  const size_t w_bins = 3 * kBins * (size_t)chunk, w_part = (size_t)(chunk * kBins * shares);
   double* dbuf = nullptr;
-  if (cudaMallocAsync((void**)&dbuf, 4 * (size_t)nb * sizeof(double), st) != cudaSuccess) {
+  if (cudaMallocAsync((void**)&dbuf, (w_bins + w_part + (size_t)nb) * sizeof(double), st) != cudaSuccess) {
     cudaGetLastError();
     return VH_E_NOMEM;
   }
-  double* dout = dbuf + 3 * nb;
+  double *part = dbuf + w_bins, *dout = part + w_part;
   const double pref = degeneracy / (8 * M_PI * M_PI * M_PI);
   int rc = VH_OK;
-  if (cudaMemcpyAsync(dbuf, bins.data(), 3 * (size_t)nb * sizeof(double), cudaMemcpyHostToDevice, st) != cudaSuccess)
-    rc = VH_E_CUDA;
-  if (rc == VH_OK) {
-    k_cooper_frye<D><<<(unsigned)nb, kThreads, 0, st>>>(el, count, dbuf, y, t_fo, pref, dout);
-    if (cudaGetLastError() != cudaSuccess ||
-        cudaMemcpyAsync(out, dout, (size_t)nb * sizeof(double), cudaMemcpyDeviceToHost, st) != cudaSuccess)
+  for (long long t0 = 0; t0 < tiles && rc == VH_OK; t0 += chunk) {
+    const int n = (int)(tiles - t0 < chunk ? tiles - t0 : chunk);
+    if (cudaMemcpyAsync(dbuf, &bins[3 * kBins * (size_t)t0], 3 * kBins * (size_t)n * sizeof(double),
+                        cudaMemcpyHostToDevice, st) != cudaSuccess) {
       rc = VH_E_CUDA;
+      break;
+    }
+    k_cooper_frye<D><<<dim3((unsigned)n, (unsigned)shares), kCfThreads, 0, st>>>(el, count, dbuf, y, t_fo, part);
+    k_cf_final<<<(unsigned)(((long long)n * kBins * 32 + 255) / 256), 256, 0, st>>>(part, (int)shares, tl, t0, n, pref,
+                                                                                    dout);
+    if (cudaGetLastError() != cudaSuccess) rc = VH_E_CUDA;
   }
+  if (rc == VH_OK &&
+      cudaMemcpyAsync(out, dout, (size_t)nb * sizeof(double), cudaMemcpyDeviceToHost, st) != cudaSuccess)
+    rc = VH_E_CUDA;
   if (cudaFreeAsync(dbuf, st) != cudaSuccess && rc == VH_OK) rc = VH_E_CUDA;
   if (cudaStreamSynchronize(st) != cudaSuccess && rc == VH_OK) rc = VH_E_CUDA;
   return rc;
