@@ -82,6 +82,57 @@ __host__ VH_HD inline long long cix(const DevCfg& C, int i, int j, int k) {
   return ((long long)k * C.gy + j) * C.px + i;
 }
 
+// ---------------------------------------------------- reciprocal and root
+// On the device, from the hardware's approximate seeds and one step of an
+// iteration for the zero of 1/r - x or 1/y^2 - s, without the general
+// division's treatment of subnormal and overflowing operands (no operand here
+// comes near them; zero and non-finite ones still give a non-finite result).
+// On the host, the plain operations.
+//
+// fast_rcp: FP64, the seed (rcp.approx.ftz.f64, about 20 bits) and one
+// third-order step r (1 + d + d^2), d = 1 - x r: the error left is d^3, below
+// the last bit.  FP32, the seed alone (1 ulp).
+#ifdef __CUDACC__
+__device__ __forceinline__ double fast_rcp(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double d = fma(-x, r, 1.0);
+  return fma(r, fma(d, d, d), r);
+}
+__device__ __forceinline__ float fast_rcp(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+#endif
+// 1/x to within an ulp (FP32: the seed and one Newton step)
+template <class R>
+VH_HD inline R rcp(R x) {
+#ifdef __CUDA_ARCH__
+  const R r = fast_rcp(x);
+  if (sizeof(R) == 8) return r;
+  return fma(r, fma(-x, r, (R)1), r);
+#else
+  return (R)1 / x;
+#endif
+}
+// sqrt(s) and 1/sqrt(s) of s >= 1: the seed (rsqrt.approx.ftz.f64), one
+// third-order step y (1 + d/2 + 3 d^2/8), d = 1 - s y^2, and a Newton
+// correction of the root
+VH_HD inline void root_rsqrt(double s, double& root, double& inv) {
+#ifdef __CUDA_ARCH__
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(s));
+  const double d = fma(-s * y, y, 1.0);
+  inv = fma(y, d * fma(0.375, d, 0.5), y);
+  const double r = s * inv;
+  root = fma(0.5 * inv, fma(-r, r, s), r);
+#else
+  root = sqrt(s);
+  inv = 1.0 / root;
+#endif
+}
+
 // ------------------------------------------------------------------ EOS
 
 template <class R>
@@ -140,7 +191,7 @@ VH_HD inline void eos_table(const DevCfg& C, R e, R* P, R* cs2, R* T) {
     return;
   }
   int i = eos_row<R>(C, te, e);
-  R w = (e - te[i]) / (te[i + 1] - te[i]);
+  R w = (e - te[i]) * rcp<R>(te[i + 1] - te[i]);
   *P = tp[i] + w * (tp[i + 1] - tp[i]);
   *cs2 = tc[i] + w * (tc[i + 1] - tc[i]);
   *T = tt[i] + w * (tt[i + 1] - tt[i]);
@@ -149,7 +200,7 @@ VH_HD inline void eos_table(const DevCfg& C, R e, R* P, R* cs2, R* T) {
 // P(e) (NEWEST5/maindef.h:332 EOS)
 template <class R>
 VH_HD inline R eos_P(const DevCfg& C, R e) {
-  if (C.eos_kind == 0) return e / (R)3;
+  if (C.eos_kind == 0) return e * (R)(1. / 3.);
   R P, c, T;
   eos_table<R>(C, e, &P, &c, &T);
   return P;
@@ -162,7 +213,7 @@ VH_HD inline R eos_cs2(const DevCfg& C, R e) {
   eos_table<R>(C, e, &P, &c, &T);
   return c;
 }
-VH_HD inline double conf_T(double x) { return pow(x, 0.25); }
+VH_HD inline double conf_T(double x) { return sqrt(sqrt(x)); }
 VH_HD inline float conf_T(float x) { return sqrtf(sqrtf(x)); }
 // T(e) (NEWEST5/maindef.h:335 FT)
 template <class R>
@@ -176,7 +227,7 @@ VH_HD inline R eos_T(const DevCfg& C, R e) {
 template <class R>
 VH_HD inline void eos_all(const DevCfg& C, R e, R& P, R& cs2, R& T) {
   if (C.eos_kind == 0) {
-    P = e / (R)3;
+    P = e * (R)(1. / 3.);
     cs2 = (R)1 / (R)3;
     T = conf_T(e / (R)C.eos_a);
     return;
@@ -187,11 +238,13 @@ VH_HD inline void eos_all(const DevCfg& C, R e, R& P, R& cs2, R& T) {
 // from a known temperature
 template <class R>
 VH_HD inline void transport_T(const DevCfg& C, R e, R P, R T, R* eta, R* taupi) {
-  R s = (e + P) / T;
+  R s = (e + P) * rcp<R>(T);
   R tg = T * (R)C.hbarc - (R)C.etas_tc;
   R etas = (R)C.etas0 + (R)C.etas1 * (tg > (R)0 ? tg : (R)0);
   *eta = etas * s;
-  *taupi = (C.taupi_kind == 1) ? (R)5 * (*eta) / (e + P) : C.taupi_kind == 2 ? (R)C.taupi_c : (R)1.5 * ((*eta) / P);
+  *taupi = (C.taupi_kind == 1)   ? (R)5 * (*eta) * rcp<R>(e + P)
+           : C.taupi_kind == 2 ? (R)C.taupi_c
+                               : (R)1.5 * ((*eta) * rcp<R>(P));
 }
 template <class R>
 VH_HD inline void transport(const DevCfg& C, R e, R P, R* eta, R* taupi) {
@@ -214,11 +267,11 @@ struct PiDep {
 template <class R>
 VH_HD inline PiDep<R> pi_dep(R u0, R u1, R u2, R u3, const R* p, R t2) {
   PiDep<R> d;
-  const R iD = (R)1 / (u0 * u0 - t2 * u3 * u3);
-  const R iu0 = (R)1 / u0;
+  const R iD = rcp<R>(u0 * u0 - t2 * u3 * u3);
+  const R iu0 = rcp<R>(u0);
   const R Q = u1 * u1 * p[0] + (R)2 * u1 * u2 * p[2] + u2 * u2 * p[1] + (R)2 * t2 * u3 * (u1 * p[3] + u2 * p[4]);
   d.tt = (Q - t2 * u3 * u3 * (p[0] + p[1])) * iD;
-  d.ee = (Q - u0 * u0 * (p[0] + p[1])) * iD / t2;
+  d.ee = (Q - u0 * u0 * (p[0] + p[1])) * iD * rcp<R>(t2);
   d.tx = (p[0] * u1 + p[2] * u2 + p[3] * u3 * t2) * iu0;
   d.ty = (p[2] * u1 + p[1] * u2 + p[4] * u3 * t2) * iu0;
   d.te = (u1 * p[3] + u2 * p[4] + t2 * u3 * d.ee) * iu0;
@@ -341,14 +394,14 @@ template <class R, bool FULL = false>
 VH_HD inline void is_kinematics(int cart, R tau, const R* u, const R du[4][4], R sig[4][4], R& theta, R acc[4]) {
   const R t2 = cart ? (R)1 : tau * tau;
   const R g[4] = {(R)1, (R)-1, (R)-1, -t2};
-  const R gi[4] = {(R)1, (R)-1, (R)-1, cart ? (R)-1 : (R)-1 / t2};
+  const R gi[4] = {(R)1, (R)-1, (R)-1, cart ? (R)-1 : -rcp<R>(t2)};
   R Dm[4][4];
 #pragma unroll
   for (int l = 0; l < 4; l++)
 #pragma unroll
     for (int a = 0; a < 4; a++) Dm[l][a] = du[l][a];
   if (!cart) {
-    const R itau = (R)1 / tau;
+    const R itau = rcp<R>(tau);
     Dm[0][3] += tau * u[3];
     Dm[3][0] += u[3] * itau;
     Dm[3][3] += u[0] * itau;
@@ -420,7 +473,7 @@ VH_HD inline void is_source_PT(const DevCfg& C, R tau, R e, R P, R T, const R* u
   R pa[4];
 #pragma unroll
   for (int v = 0; v < 4; v++) pa[v] = pi[v][0] * acc[0] + pi[v][1] * acc[1] + pi[v][2] * acc[2] + pi[v][3] * acc[3];
-  const R iu0 = (R)1 / u[0], itp = (R)1 / tp, itau = cart ? (R)1 : (R)1 / tau;
+  const R iu0 = rcp<R>(u[0]), itp = rcp<R>(tp), itau = cart ? (R)1 : rcp<R>(tau);
   R divv = 0;
 #pragma unroll
   for (int i = 1; i < 4; i++) divv += du[i][i] * iu0 - u[i] * du[0][i] * (iu0 * iu0);
@@ -453,7 +506,7 @@ VH_HD inline void is_source(const DevCfg& C, R tau, R e, const R* u, const R* p,
 // P and dP/de together (one table lookup)
 template <class R>
 VH_HD inline void eos_P_cs2(const DevCfg& C, R e, R& P, R& cs2) {
-  if (C.eos_kind == 0) { P = e / (R)3; cs2 = (R)1 / (R)3; return; }
+  if (C.eos_kind == 0) { P = e * (R)(1. / 3.); cs2 = (R)1 / (R)3; return; }
   R T;
   eos_table<R>(C, e, &P, &cs2, &T);
 }
@@ -471,14 +524,14 @@ VH_HD inline void c2p_fj(const DevCfg& C, const double* Tt, const double* p, dou
   const double W = Tt[0], X = Tt[1], Y = Tt[2], Z = Tt[3];
   const double p1 = p[0], p2 = p[1], p3 = p[2], p4 = p[3], p5 = p[4];
   const double S = 1 + u1 * u1 + u2 * u2 + t2 * u3 * u3;
-  const double u0 = sqrt(S);
+  double u0, iu;
+  root_rsqrt(S, u0, iu);
   const double ep = e + P;
   y[0] = (W - e) * u0 - X * u1 - Y * u2 - t2 * Z * u3;
   y[1] = X * u0 - e * u1 - u1 * (P + p1 + ep * u1 * u1) - u2 * (p3 + ep * u1 * u2) - t2 * u3 * (p4 + ep * u1 * u3);
   y[2] = Y * u0 - e * u2 - u1 * (p3 + ep * u1 * u2) - u2 * (P + p2 + ep * u2 * u2) - t2 * u3 * (p5 + ep * u2 * u3);
   y[3] = Z * u0 - p4 * u1 - p5 * u2 - u3 * (P + W - p1 - p2);
   if (!jac) return;
-  const double iu = 1.0 / u0;
   J[0][0] = -u0;
   J[0][1] = (W - e) * u1 * iu - X;
   J[0][2] = (W - e) * u2 * iu - Y;
@@ -537,6 +590,61 @@ VH_HD inline bool solve4(double A[4][4], double b[4]) {
   return true;
 }
 
+// The same without row exchanges, which in registers cost two selects per
+// entry and candidate (a third of the update kernel's instructions were
+// theirs): false, with A and b spoilt, where a multiplier exceeds 1024 and
+// the exchange is worth having.  The Jacobian is dominated by its diagonal at
+// ordinary velocities; multipliers below 1024 leave a Newton step 1e-7 of its
+// length uncertain at the very worst, and the last step is below 1e-8.
+VH_HD inline bool solve4_direct(double A[4][4], double b[4]) {
+  bool ok = true;
+#pragma unroll
+  for (int c = 0; c < 4; c++) {
+    const double ip = rcp(A[c][c]);
+    A[c][c] = ip;
+#pragma unroll
+    for (int r = c + 1; r < 4; r++) {
+      const double m = A[r][c] * ip;
+#ifdef __CUDA_ARCH__
+      ok &= (__double2hiint(m) & 0x7fffffff) <= 0x40900000;  // |m| <= 1024, false for NaN
+#else
+      ok &= fabs(m) <= 1024.0;
+#endif
+#pragma unroll
+      for (int k = c + 1; k < 4; k++) A[r][k] -= m * A[c][k];
+      b[r] -= m * b[c];
+    }
+  }
+#pragma unroll
+  for (int c = 3; c >= 0; c--) {
+    double s = b[c];
+#pragma unroll
+    for (int k = c + 1; k < 4; k++) s -= A[c][k] * b[k];
+    b[c] = s * A[c][c];
+  }
+  return ok && isfinite(b[0]) && isfinite(b[1]) && isfinite(b[2]) && isfinite(b[3]);
+}
+// The Newton step at x by elimination with row exchanges; out of line, since
+// few cells take it, and by value, so that the caller's state stays in
+// registers.
+struct NewtonStep {
+  double s0, s1, s2, s3;
+  bool ok;
+};
+#ifdef __CUDACC__
+__noinline__
+#endif
+static VH_HD NewtonStep newton_step_pivoted(const DevCfg& C, double T0, double T1, double T2, double T3, double p0,
+                                            double p1, double p2, double p3, double p4, double t2, double x0,
+                                            double x1, double x2, double x3) {
+  const double Tt[4] = {T0, T1, T2, T3}, p[5] = {p0, p1, p2, p3, p4}, x[4] = {x0, x1, x2, x3};
+  double y[4], J[4][4];
+  c2p_fj(C, Tt, p, t2, x, y, J, true);
+  double st[4] = {-y[0], -y[1], -y[2], -y[3]};
+  const bool ok = solve4(J, st);
+  return {st[0], st[1], st[2], st[3], ok};
+}
+
 // Newton with norm-reducing step control and the reference's form of
 // stopping rule (|dx_i| < rtol |x_i| or dx_i = 0 for all i, at most 100
 // iterations; NEWEST5/multiroot.h:389-422, where rtol = 1e-16).  A step that
@@ -573,7 +681,15 @@ VH_HD inline int con2prim(const DevCfg& C, const double* Tt, const double* p, do
   while (it < 100) {
     it++;
     double st[4] = {-y[0], -y[1], -y[2], -y[3]};
-    if (!solve4(J, st)) return -1;
+    if (!solve4_direct(J, st)) {
+      const NewtonStep n = newton_step_pivoted(C, Tt[0], Tt[1], Tt[2], Tt[3], p[0], p[1], p[2], p[3], p[4], t2, x[0],
+                                               x[1], x[2], x[3]);
+      if (!n.ok) return -1;
+      st[0] = n.s0;
+      st[1] = n.s1;
+      st[2] = n.s2;
+      st[3] = n.s3;
+    }
     if (qskip > 0.0) {
       bool small = true;
 #pragma unroll

@@ -101,10 +101,12 @@ struct CellAt {
   long long c;
 };
 __device__ __forceinline__ CellAt cell_at(const DevCfg& C, long long t) {
+  // 32-bit division: a handle's arrays would not fit the GPU at 2^31 cells
+  const unsigned row = (unsigned)t / (unsigned)C.nx, k = row / (unsigned)C.ny;
   CellAt x;
-  x.i = C.il + (int)(t % C.nx);
-  x.j = C.jl + (int)((t / C.nx) % C.ny);
-  x.k = C.kl + (int)(t / ((long long)C.nx * C.ny));
+  x.i = C.il + (int)((unsigned)t - row * (unsigned)C.nx);
+  x.j = C.jl + (int)(row - k * (unsigned)C.ny);
+  x.k = C.kl + (int)k;
   x.c = cix(C, x.i, x.j, x.k);
   return x;
 }
@@ -354,17 +356,22 @@ __device__ __forceinline__ unsigned update_cell(const DevCfg& C, const DevPtrs<R
   return root_cell<R, STAGE>(C, P, tau_n, ts, x, e, u, pu, q9, t_gev);
 }
 
-// one thread per interior cell.  Blocks per SM: FP64 4 (128 registers),
-// mixed 5 (96 registers); measured on the 161x161x41 event, FP64 per step
-// 1.671 / 1.719 / 1.775 / 1.797 ms at 4 / 5 / 6 / 7 blocks (fewer spills
-// win), mixed 0.975 / 0.957 / 0.977 / 0.977 ms
+// One thread per interior cell.  Bound by the latency of its loads and of the
+// Newton chain, with DRAM at half its rate (88 words a cell and launch in
+// 3+1D).  Blocks per SM: FP64 4 (128 registers), mixed 5 (96); measured on the
+// 161x161x41 event, ms per stage-1 launch: FP64 0.220 / 0.213 / 0.305 at 3 / 4 /
+// 5 blocks (spills), mixed 0.155 / 0.146 / 0.145 at 4 / 5 / 6.  Divisions and
+// roots by the hardware's seeds and one step (rcp, root_rsqrt), elimination
+// without row exchanges and the asynchronous prefetch brought it from 0.273 /
+// 0.193 (and 0.211 / 0.138 before the directions had a divergence set each).
 constexpr int kUpdThreads = 128;
 template <class R>
 struct UpdOcc {
   static constexpr int MIN_BLOCKS = sizeof(R) == 8 ? 4 : 5;
 };
 template <class R, int STAGE>
-__global__ void __launch_bounds__(kUpdThreads, UpdOcc<R>::MIN_BLOCKS) k_update(DevCfg C, DevPtrs<R> P, double tau_n, double ts) {
+__global__ void __launch_bounds__(kUpdThreads, UpdOcc<R>::MIN_BLOCKS) k_update(const __grid_constant__ DevCfg C, const __grid_constant__ DevPtrs<R> P, double tau_n,
+                                                                                        double ts) {
   pdl_wait_then_release();
   if (*P.status) return;
   const long long nint = (long long)C.nx * C.ny * (C.kr - C.kl);

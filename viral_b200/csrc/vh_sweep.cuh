@@ -133,24 +133,6 @@ __device__ __forceinline__ D2 v_pair(double a, double b) { return {a, b}; }
 __device__ __forceinline__ void v_split(F2 x, float& a, float& b) { f2u(x, a, b); }
 __device__ __forceinline__ void v_split(D2 x, double& a, double& b) { a = x.a; b = x.b; }
 
-// 1/x for finite x well inside the normal range.  FP64: the hardware's seed
-// (rcp.approx.ftz.f64, about 20 bits) refined by one third-order Newton-type
-// step, r (1 + d + d^2) with d = 1 - x r: the error left is d^3, below the
-// last bit.  x here is a product of up to four sums of WENO weights, between
-// about 1e-92 and 1e160 for any state the step takes, so no special case of
-// the general division applies.  FP32: the hardware's reciprocal (1 ulp).
-__device__ __forceinline__ double fast_rcp(double x) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  const double d = fma(-x, r, 1.0);
-  return fma(r, fma(d, d, d), r);
-}
-__device__ __forceinline__ float fast_rcp(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-
 // ------------------------------------------------------------------ WENO5
 // The face values of a stencil (vh_device.cuh, weno_lr) in difference form.
 // With the first differences dm = q_c - q_{c-1}, dp = q_{c+1} - q_c and the
@@ -204,7 +186,7 @@ __device__ __forceinline__ void cell_flux(const DevCfg& C, R tau, R e, const R* 
   const R ep = e + P;
   const R u0 = u[0], u1 = u[1], u2 = u[2], u3 = u[3];
   const PiDep<R> d = pi_dep<R>(u0, u1, u2, u3, p, t2);
-  const R iu0 = (R)1 / u0;
+  const R iu0 = rcp<R>(u0);
   if (DIR == 0) {
     F[0] = tf * (d.tx + u1 * u0 * ep);
     F[1] = tf * (p[0] + P + u1 * u1 * ep);
@@ -221,7 +203,7 @@ __device__ __forceinline__ void cell_flux(const DevCfg& C, R tau, R e, const R* 
     F[0] = tf * (d.te + u3 * u0 * ep);
     F[1] = tf * (p[3] + u3 * u1 * ep);
     F[2] = tf * (p[4] + u3 * u2 * ep);
-    F[3] = cart ? (d.ee + P + u3 * u3 * ep) : tf * (d.ee + P / t2 + u3 * u3 * ep);
+    F[3] = cart ? (d.ee + P + u3 * u3 * ep) : tf * (d.ee + P * rcp<R>(t2) + u3 * u3 * ep);
     // the eta flux of pi and its speed carry a factor tau (NEWEST5/hydroKT.h:76-81)
     v = cart ? u3 * iu0 : tau * u3 * iu0;
   }
