@@ -156,23 +156,12 @@ extern "C" int vh_dims(const vh_handle* h, int* gx, int* gy, int* gz) {
 
 // canonical doubles (18 fields; host or device) -> state
 static int import_state(vh_handle* h, const double* canon) {
-  const long long n18 = 18 * h->C.n;
-  if (h->mixed) {
-    if (int r = pitched_in(h, h->stage, canon, 18)) return r;
-    k_d2f<<<grid1(n18, 256), 256, 0, h->stream>>>(h->stage, static_cast<float*>(h->state), n18);
-  } else if (canon != h->state) {
-    if (int r = pitched_in(h, static_cast<double*>(h->state), canon, 18)) return r;
-  }
-  VH_CUDA(h, cudaGetLastError());
-  return VH_OK;
+  if (h->mixed) return pitched_in(h, static_cast<float*>(h->state), canon, 18);
+  if (canon == h->state) return VH_OK;
+  return pitched_in(h, static_cast<double*>(h->state), canon, 18);
 }
 static int export_state(vh_handle* h, double* canon) {
-  const long long n18 = 18 * h->C.n;
-  if (h->mixed) {
-    k_f2d<<<grid1(n18, 256), 256, 0, h->stream>>>(static_cast<const float*>(h->state), h->stage, n18);
-    VH_CUDA(h, cudaGetLastError());
-    return pitched_out(h, canon, h->stage, 18);
-  }
+  if (h->mixed) return pitched_out(h, canon, static_cast<const float*>(h->state), 18);
   return pitched_out(h, canon, static_cast<const double*>(h->state), 18);
 }
 

@@ -410,14 +410,4 @@ __global__ void k_cfl(DevCfg C, DevPtrs<R> P, double tau, unsigned long long* ou
   if ((threadIdx.x & 31) == 0) atomic_max_nonneg(out, m);
 }
 
-// precision conversion between the canonical double layout and float state
-static __global__ void k_d2f(const double* in, float* out, long long n) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < n) out[t] = (float)in[t];
-}
-static __global__ void k_f2d(const float* in, double* out, long long n) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < n) out[t] = (double)in[t];
-}
-
 }  // namespace vh
