@@ -293,10 +293,10 @@ struct DirArgs {
   R* out;        // 2 x 10 fields: line adjoints (x lines, then y lines)
 };
 
-// quantities whose WENO stencils are reversed at the same time, threads per
-// line block, and shared-memory words per line cell
-constexpr int kQP = 4;
-constexpr int kDirWords = 55 + 5 * kQP;
+// shared-memory words per line cell, the last ones for the reversed segments'
+// edges
+constexpr int kEdgeWords = 16;
+constexpr int kDirWords = 55 + kEdgeWords;
 // threads per line block: two blocks per SM keep all the lines of a 128^2
 // grid (256 blocks) resident in one wave at either precision
 template <class R>
@@ -320,7 +320,7 @@ __device__ __forceinline__ void adj_line(const DirArgs<R>& a, int line, R* sm) {
   const long long stride = DIR == 0 ? 1 : C.px;
   const long long base = DIR == 0 ? cix(C, 0, C.jl + line, 0) : cix(C, C.il + line, 0, 0);
   const double hh = DIR == 0 ? C.dx : C.dy;
-  const R h = (R)hh, inv_h = (R)(1.0 / hh);
+  const R inv_h = (R)(1.0 / hh);
   R* q = sm;            // 13: flux quantities
   R* lv = q + 13 * G;   // 7: face state at the right face (V^0..5, speed)
   R* rv = lv + 7 * G;   // 7: face state at the left face
@@ -330,7 +330,7 @@ __device__ __forceinline__ void adj_line(const DirArgs<R>& a, int line, R* sm) {
   R* sr = sl + G;       // adjoint of the speed's left-face state
   R* qb = sr + G;       // 16: adjoints of the 13 quantities and of u^0..2
   R* uu = qb + 16 * G;  // 3: u^0..2 along the line
-  R* c5 = uu + 3 * G;   // 5 x kQP: stencil contributions of the quantities in flight
+  R* edge = uu + 3 * G; // weno_reverse's edges
   const int tid = threadIdx.x, nt = blockDim.x;
 
   for (int i = tid; i < G; i += nt) {
@@ -376,15 +376,14 @@ __device__ __forceinline__ void adj_line(const DirArgs<R>& a, int line, R* sm) {
     }
   }
   __syncthreads();
-  // WENO stencils in reverse, kQP quantities at a time (the 13 flux
-  // quantities, then the three velocity lines of the derivative du^l/dx)
-  for (int k0 = 0; k0 < 16; k0 += kQP) {
-    for (int w = tid; w < kQP * G; w += nt) {
-      const int kq = w / G, i = w % G, k = k0 + kq;
-      R cc[5] = {0, 0, 0, 0, 0};
-      if (k < 16 && i >= lo - 1 && i <= hi) {
+  // WENO stencils in reverse: the 13 flux quantities, then the three velocity
+  // lines of the derivative du^l/dx
+  weno_reverse<R, 16>(
+      G, lo, hi, qb, edge, kEdgeWords * G, [&](int k) { return k < 13 ? q + k * G : uu + (k - 13) * G; },
+      [&](int k, int i, R& Lb, R& Rb) {
         const bool hasL = i <= hi - 1, hasR = i >= lo;  // faces i and i-1
-        R Lb = 0, Rb = 0;
+        Lb = 0;
+        Rb = 0;
         if (k < 6) {
           if (hasL) Lb = (R)0.5 * hb[k * G + i];
           if (hasR) Rb = (R)0.5 * hb[k * G + i - 1];
@@ -395,29 +394,10 @@ __device__ __forceinline__ void adj_line(const DirArgs<R>& a, int line, R* sm) {
           Lb = sl[i];
           Rb = sr[i];
         } else if (i >= lo && i < hi) {
-          const R d = a.dub[((k - 13) * 2 + DIR) * n + base + i * stride];
-          Lb = d / h;
-          Rb = -d / h;
+          Lb = a.dub[((k - 13) * 2 + DIR) * n + base + i * stride] * inv_h;
+          Rb = -Lb;
         }
-        const R* s = k < 13 ? q + k * G : uu + (k - 13) * G;
-        if (Lb != (R)0 || Rb != (R)0) weno_lr_vjp<R>(s + i - 2, Lb, Rb, cc);
-      }
-#pragma unroll
-      for (int o = 0; o < 5; o++) c5[(kq * 5 + o) * G + i] = cc[o];
-    }
-    __syncthreads();
-    for (int w = tid; w < kQP * G; w += nt) {
-      const int kq = w / G, jj = w % G, k = k0 + kq;
-      R acc = 0;
-#pragma unroll
-      for (int o = 0; o < 5; o++) {
-        const int i = jj + 2 - o;
-        if (i >= 0 && i < G) acc += c5[(kq * 5 + o) * G + i];
-      }
-      if (k < 16) qb[k * G + jj] += acc;
-    }
-    __syncthreads();
-  }
+      });
   for (int jj = tid; jj < G; jj += nt) {
     const long long c = base + jj * stride;
     R x[NX], qbl[NQ], xb[NX];

@@ -108,7 +108,7 @@ VH_HD inline void weno_lr_vjp(const R* q, R Lbar, R Rbar, R* qbar) {
     const R nl[3] = {(R)0.3 * P12, (R)0.6 * P02, (R)0.1 * P01}, nr[3] = {(R)0.1 * P12, (R)0.6 * P02, (R)0.3 * P01};
     const R numl = nl[0] * ql[0] + nl[1] * ql[1] + nl[2] * ql[2], denl = (R)6 * (nl[0] + nl[1] + nl[2]);
     const R numr = nr[0] * qr[0] + nr[1] * qr[1] + nr[2] * qr[2], denr = (R)6 * (nr[0] + nr[1] + nr[2]);
-    const R inv = (R)1 / (denl * denr), idl = denr * inv, idr = denl * inv;
+    const R inv = rcp<R>(denl * denr), idl = denr * inv, idr = denl * inv;
     const R numlb = Lbar * idl, denlb = -Lbar * numl * idl * idl;
     const R numrb = Rbar * idr, denrb = -Rbar * numr * idr * idr;
     R nlb[3], nrb[3];

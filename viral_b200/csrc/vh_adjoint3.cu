@@ -297,14 +297,11 @@ struct Dir3Args {
   R* out;        // 3 x 14 fields: line adjoints (x lines, y lines, eta lines)
 };
 
-// quantities whose WENO stencils are reversed at the same time, and
-// shared-memory words per line cell: flux quantities 19, flux adjoints 9,
-// max speed 1, speed-state adjoints 2, quantity adjoints 23, velocities 4,
-// and one region used first for the face states (2 x 10) and then for the
-// stencil contributions (5 per quantity in flight)
-constexpr int kQP3 = 4;
-constexpr int kDir3Shared = 5 * kQP3 > 20 ? 5 * kQP3 : 20;
-constexpr int kDir3Words = NQ3 + 9 + 1 + 2 + KQ3 + NVEL + kDir3Shared;
+// shared-memory words per line cell: flux quantities 19, flux adjoints 9, max
+// speed 1, speed-state adjoints 2, quantity adjoints 23, velocities 4, and one
+// region used first for the face states (2 x 10) and then for the reversed
+// segments' edges
+constexpr int kDir3Words = NQ3 + 9 + 1 + 2 + KQ3 + NVEL + 20;
 
 template <class R>
 __device__ __forceinline__ R sgn3(R x) { return (R)((x > (R)0) - (x < (R)0)); }
@@ -323,7 +320,7 @@ __device__ __forceinline__ void adj_line3(const Dir3Args<R>& a, int line, R* sm)
   else if (DIR == 1) base = cix(C, C.il + line % C.nx, 0, C.kl + line / C.nx);
   else base = cix(C, C.il + line % C.nx, C.jl + line / C.nx, 0);
   const double hh = DIR == 0 ? C.dx : (DIR == 1 ? C.dy : C.dz);
-  const R h = (R)hh, inv_h = (R)(1.0 / hh);
+  const R inv_h = (R)(1.0 / hh);
   R* q = sm;              // 19: flux quantities
   R* hb = q + NQ3 * G;    // 9: adjoint of the KT flux at the face right of cell f
   R* am = hb + 9 * G;     // max signal speed at that face
@@ -333,8 +330,7 @@ __device__ __forceinline__ void adj_line3(const Dir3Args<R>& a, int line, R* sm)
   R* uu = qb + KQ3 * G;   // 4: u^0..3 along the line
   R* lv = uu + NVEL * G;  // 10: face state at the right face (V^0..8, speed)
   R* rv = lv + 10 * G;    // 10: face state at the left face
-  R* c5 = lv;             // 5 x kQP3: stencil contributions of the quantities in
-                          // flight (after the face states are used)
+  R* edge = lv;           // weno_reverse's edges (after the face states are used)
   const int tid = threadIdx.x, nt = blockDim.x;
 
   for (int i = tid; i < G; i += nt) {
@@ -380,15 +376,14 @@ __device__ __forceinline__ void adj_line3(const Dir3Args<R>& a, int line, R* sm)
     }
   }
   __syncthreads();
-  // WENO stencils in reverse, kQP3 quantities at a time (the 19 flux
-  // quantities, then the four velocity lines of the derivative du^l/dx^DIR)
-  for (int k0 = 0; k0 < KQ3; k0 += kQP3) {
-    for (int w = tid; w < kQP3 * G; w += nt) {
-      const int kq = w / G, i = w % G, k = k0 + kq;
-      R cc[5] = {0, 0, 0, 0, 0};
-      if (k < KQ3 && i >= lo - 1 && i <= hi) {
+  // WENO stencils in reverse: the 19 flux quantities, then the four velocity
+  // lines of the derivative du^l/dx^DIR
+  weno_reverse<R, KQ3>(
+      G, lo, hi, qb, edge, 20 * G, [&](int k) { return k < NQ3 ? q + k * G : uu + (k - NQ3) * G; },
+      [&](int k, int i, R& Lb, R& Rb) {
         const bool hasL = i <= hi - 1, hasR = i >= lo;  // faces i and i-1
-        R Lb = 0, Rb = 0;
+        Lb = 0;
+        Rb = 0;
         if (k < 9) {
           if (hasL) Lb = (R)0.5 * hb[k * G + i];
           if (hasR) Rb = (R)0.5 * hb[k * G + i - 1];
@@ -399,29 +394,10 @@ __device__ __forceinline__ void adj_line3(const Dir3Args<R>& a, int line, R* sm)
           Lb = sl[i];
           Rb = sr[i];
         } else if (i >= lo && i < hi) {
-          const R d = a.dub[((k - NQ3) * 3 + DIR) * n + base + i * stride];
-          Lb = d / h;
-          Rb = -d / h;
+          Lb = a.dub[((k - NQ3) * 3 + DIR) * n + base + i * stride] * inv_h;
+          Rb = -Lb;
         }
-        const R* s = k < NQ3 ? q + k * G : uu + (k - NQ3) * G;
-        if (Lb != (R)0 || Rb != (R)0) weno_lr_vjp<R>(s + i - 2, Lb, Rb, cc);
-      }
-#pragma unroll
-      for (int o = 0; o < 5; o++) c5[(kq * 5 + o) * G + i] = cc[o];
-    }
-    __syncthreads();
-    for (int w = tid; w < kQP3 * G; w += nt) {
-      const int kq = w / G, jj = w % G, k = k0 + kq;
-      R acc = 0;
-#pragma unroll
-      for (int o = 0; o < 5; o++) {
-        const int i = jj + 2 - o;
-        if (i >= 0 && i < G) acc += c5[(kq * 5 + o) * G + i];
-      }
-      if (k < KQ3) qb[k * G + jj] += acc;
-    }
-    __syncthreads();
-  }
+      });
   for (int jj = tid; jj < G; jj += nt) {
     const long long c = base + jj * stride;
     R x[NX3], qbl[NQ3], xb[NX3];
@@ -447,8 +423,8 @@ __global__ void __launch_bounds__(256) k_adj3_dir(Dir3Args<R> a) {
 }
 
 // line length, line count, threads and shared memory of the lines along d:
-// 256 threads per line along x and y; along eta, where lines are short and
-// many, the line length rounded up to warps (at most 256); shared memory for
+// 256 threads per line (11 segments for each of the 23 quantities), 128 for
+// lines of up to 64 cells, as those along eta usually are; shared memory for
 // that line length only
 struct LineShape {
   int G;
@@ -461,7 +437,7 @@ LineShape line_shape(const DevCfg& C, int d) {
   LineShape s;
   s.G = d == 0 ? C.gx : (d == 1 ? C.gy : C.gz);
   s.lines = d == 0 ? (long long)C.ny * C.nz : (d == 1 ? (long long)C.nx * C.nz : (long long)C.nx * C.ny);
-  s.threads = d == 2 ? std::min(256, (s.G + 31) / 32 * 32) : 256;
+  s.threads = s.G <= 64 ? 128 : 256;
   s.smem = (size_t)kDir3Words * s.G * sizeof(R);
   return s;
 }

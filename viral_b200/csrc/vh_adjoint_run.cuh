@@ -146,6 +146,57 @@ static int eps_p_device(vh_handle* h, const R* S, double* part, double* nd_dev, 
 }
 
 
+// Reverse of the WENO stencils of K quantities along a line of G cells in
+// shared memory (stencil centres lo-1 .. hi): qb[k*G + i] becomes the adjoint
+// of quantity k at cell i.  The block's threads are K tasks x S segments of
+// the line; a thread walks its segment's centres with the stencil and the
+// adjoints of the cells under it in registers, writes the cells that are
+// complete and leaves two cells' worth on either side in `edge`, added after
+// one barrier.  Segments hold four centres at least, so that no cell takes
+// from two neighbours at once.  The stencils of four quantities at a time
+// through shared memory, with two barriers each, had left the block at
+// barriers for a quarter of its time.  src(k): quantity k's line; lr(k, i, L,
+// R): the adjoints of its two face values at centre i.  Ends in a barrier.
+template <class R, int K, class Src, class Lr>
+__device__ __forceinline__ void weno_reverse(int G, int lo, int hi, R* qb, R* edge, int edge_words, Src&& src, Lr&& lr) {
+  const int m = hi - lo + 2, nt = blockDim.x, tid = threadIdx.x;
+  const int S = max(1, min(nt / K, min(m / 4, edge_words / (4 * K))));
+  const int k = tid / S, seg = tid % S;
+  if (k < K) {
+    const int c0 = lo - 1 + m * seg / S, c1 = lo - 1 + m * (seg + 1) / S;
+    const R* s = src(k);
+    R* e = edge + (k * S + seg) * 4;
+    R* out = qb + k * G;
+    R w[5] = {s[c0 - 2], s[c0 - 1], s[c0], s[c0 + 1], 0}, acc[4] = {0, 0, 0, 0};
+    for (int i = c0; i < c1; i++) {
+      w[4] = s[i + 2];
+      R L, Rr, cc[5] = {0, 0, 0, 0, 0};
+      lr(k, i, L, Rr);
+      if (L != (R)0 || Rr != (R)0) weno_lr_vjp<R>(w, L, Rr, cc);
+      const R done = acc[0] + cc[0];  // cell i - 2
+      if (i - 2 >= c0) out[i - 2] = done;
+      else e[i - c0] = done;
+      acc[0] = acc[1] + cc[1];
+      acc[1] = acc[2] + cc[2];
+      acc[2] = acc[3] + cc[3];
+      acc[3] = cc[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) w[q] = w[q + 1];
+    }
+    out[c1 - 2] = acc[0];
+    out[c1 - 1] = acc[1];
+    e[2] = acc[2];
+    e[3] = acc[3];
+  }
+  __syncthreads();
+  for (int x = tid; x < K * S * 4; x += nt) {
+    const int q = x & 3, sg = (x >> 2) % S, kk = (x >> 2) / S;
+    const int cell = q < 2 ? lo - 1 + m * sg / S - 2 + q : lo - 1 + m * (sg + 1) / S + q - 2;
+    qb[kk * G + cell] += edge[x];
+  }
+  __syncthreads();
+}
+
 // the 3+1D discrete adjoint (vh_adjoint3.cu)
 int adjoint3_eps_p(vh_handle* h, int nsteps, int every, double* eps_p, double* grad_state, double* grad_e,
                    double* grad_etas);
