@@ -206,13 +206,6 @@ __global__ void k_barrier_probe(unsigned int* bar, int absent) {
   grid_barrier(bar, 1ll << 20);
 }
 
-// copy one event's canonical doubles (18 x n) into its pool view
-template <class R>
-__global__ void k_import_event(const double* src, DevPtrs<R> P, long long n) {
-  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= n) return;
-  for (int q = 0; q < 18; q++) P.f(q)[c] = (R)src[q * n + c];
-}
 template <class R>
 __global__ void k_export_event(DevPtrs<R> P, double* dst, long long n) {
   const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -437,13 +430,40 @@ extern "C" int vh_batch_destroy(vh_batch* b) {
   return VH_OK;
 }
 
+// the canonical fields of an event from its profile: e, u^x, u^y at src, then
+// prevu (4) and pi (5) where given; u^eta = 0, T^{tau mu} follows
 template <class R>
-static int import_event(vh_batch* b, int ev, const double* host18, int pi_mode) {
+__global__ void k_import_profile(const double* src, int prevu, int pi, DevPtrs<R> P, long long n) {
+  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= n) return;
+  const double ux = src[n + c], uy = src[2 * n + c];
+  // rounded product by product, as a host compiler without contraction does
+  const double u[4] = {sqrt(__dadd_rn(__dadd_rn(1.0, __dmul_rn(ux, ux)), __dmul_rn(uy, uy))), ux, uy, 0.0};
+  P.e()[c] = (R)src[c];
+  for (int l = 0; l < 4; l++) {
+    P.u(l)[c] = (R)u[l];
+    P.pu(l)[c] = (R)(prevu ? src[(3 + l) * n + c] : u[l]);
+    P.A(l)[c] = 0;
+  }
+  const double* p = src + (prevu ? 7 : 3) * n;
+  for (int l = 0; l < 5; l++) P.A(4 + l)[c] = pi ? (R)p[l * n + c] : (R)0;
+}
+
+template <class R>
+static int import_event(vh_batch* b, int ev, const double* e, const double* ux, const double* uy, const double* prevu4,
+                        int pi_mode, const double* pi5) {
   const long long n = (long long)(b->nx[ev] + 6) * (b->ny[ev] + 6);
-  VB_CUDA(b, cudaMemcpy(b->stage, host18, sizeof(double) * 18 * n, cudaMemcpyHostToDevice));
+  const size_t nb = sizeof(double) * (size_t)n;
+  // the caller's arrays as they are; 12 fields at most, the staging has 18
+  VB_CUDA(b, cudaMemcpyAsync(b->stage, e, nb, cudaMemcpyDefault, nullptr));
+  VB_CUDA(b, cudaMemcpyAsync(b->stage + n, ux, nb, cudaMemcpyDefault, nullptr));
+  VB_CUDA(b, cudaMemcpyAsync(b->stage + 2 * n, uy, nb, cudaMemcpyDefault, nullptr));
+  if (prevu4) VB_CUDA(b, cudaMemcpyAsync(b->stage + 3 * n, prevu4, 4 * nb, cudaMemcpyDefault, nullptr));
+  const bool pi = pi_mode == VH_PI_GIVEN;
+  if (pi) VB_CUDA(b, cudaMemcpyAsync(b->stage + (prevu4 ? 7 : 3) * n, pi5, 5 * nb, cudaMemcpyDefault, nullptr));
   DevPtrs<R> P = pool_ptrs<R>(b).shifted(b->off[ev]);
   P.status = b->d_flag + ev;
-  k_import_event<R><<<(unsigned)((n + 255) / 256), 256>>>(b->stage, P, n);
+  k_import_profile<R><<<(unsigned)((n + 255) / 256), 256>>>(b->stage, prevu4 != nullptr, pi, P, n);
   DevCfg C = b->C0;
   C.nx = b->nx[ev]; C.ny = b->ny[ev]; C.gx = C.nx + 6; C.gy = C.ny + 6; C.px = C.gx; C.xt0 = 3; C.ir = 3 + C.nx; C.jr = 3 + C.ny;
   C.il = C.jl = 3; C.n = n;
@@ -463,17 +483,8 @@ extern "C" int vh_batch_init_event(vh_batch* b, int ev, const double* e, const d
   if (!b || ev < 0 || ev >= b->n || !e || !ux || !uy) return VH_E_ARG;
   if (pi_mode != VH_PI_GIVEN && pi_mode != VH_PI_ZERO && pi_mode != VH_PI_NS) return VH_E_ARG;
   if (pi_mode == VH_PI_GIVEN && !pi5) return VH_E_ARG;
-  const long long n = (long long)(b->nx[ev] + 6) * (b->ny[ev] + 6);
-  std::vector<double> f(18 * (size_t)n, 0.0);
-  for (long long c = 0; c < n; c++) {
-    f[c] = e[c];
-    f[2 * n + c] = ux[c];
-    f[3 * n + c] = uy[c];
-    f[n + c] = std::sqrt(1 + ux[c] * ux[c] + uy[c] * uy[c]);
-    for (int l = 0; l < 5; l++) f[(5 + l) * n + c] = pi_mode == VH_PI_GIVEN ? pi5[l * n + c] : 0.0;
-    for (int l = 0; l < 4; l++) f[(14 + l) * n + c] = prevu4 ? prevu4[l * n + c] : f[(1 + l) * n + c];
-  }
-  return b->mixed ? import_event<float>(b, ev, f.data(), pi_mode) : import_event<double>(b, ev, f.data(), pi_mode);
+  return b->mixed ? import_event<float>(b, ev, e, ux, uy, prevu4, pi_mode, pi5)
+                  : import_event<double>(b, ev, e, ux, uy, prevu4, pi_mode, pi5);
 }
 
 // Glauber events for every slot, generated on host threads (vh_profile_glauber

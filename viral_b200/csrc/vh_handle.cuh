@@ -13,6 +13,7 @@
 
 #include "vh.h"
 #include "vh_aux.cuh"
+#include "vh_hostcopy.cuh"
 #include "vh_nvtx.h"
 
 using namespace vh;
@@ -59,6 +60,7 @@ struct vh_handle {
   // device arrays (allocated on first use)
   double* xfer = nullptr;
   size_t xfer_bytes = 0;
+  HostCopy to_host;  // large results into pageable memory
   std::string err;
 };
 
@@ -314,7 +316,7 @@ static int pitched_out(vh_handle* h, double* canon, const R* dev_padded, int nfi
   const DevCfg& C = h->C;
   const long long nc = canon_cells(C), total = nfields * nc;
   if (sizeof(R) == 8 && C.px == C.gx) {
-    VH_CUDA(h, cudaMemcpyAsync(canon, dev_padded, sizeof(double) * total, cudaMemcpyDefault, h->stream));
+    VH_CUDA(h, h->to_host.copy(canon, dev_padded, sizeof(double) * total, h->stream));
     return VH_OK;
   }
   const bool dev = device_accessible(canon);
@@ -324,7 +326,7 @@ static int pitched_out(vh_handle* h, double* canon, const R* dev_padded, int nfi
   k_repitch<R, false><<<dim3(grid1(nc, 1024), nfields), 256, 0, h->stream>>>(x, dev_padded, (unsigned)nc, C.n,
                                                                              (unsigned)C.gx, (unsigned)C.px);
   VH_CUDA(h, cudaGetLastError());
-  if (!dev) VH_CUDA(h, cudaMemcpyAsync(canon, x, sizeof(double) * total, cudaMemcpyDeviceToHost, h->stream));
+  if (!dev) VH_CUDA(h, h->to_host.copy(canon, x, sizeof(double) * total, h->stream));
   return VH_OK;
 }
 
