@@ -292,10 +292,9 @@ __device__ __forceinline__ bool tile_by_tma(const DevPtrs<R>& P, const SweepLay<
 
 // A thread owns two quantities, F^l and V^l (tasks 0..8) or two components of
 // u^mu (9, 10).
-template <class R, int DIR, bool MM, bool TMA>
-__device__ __forceinline__ void walk(const DevCfg& C, const DevPtrs<R>& P, const SweepLay<R, DIR>& L, R* sm,
-                                          int so, int sp, int sa, int tid, int nout, R inv_h, bool ok,
-                                          long long cell0, long long stride) {
+template <class R, int DIR, bool TMA>
+__device__ __forceinline__ void walk(const DevPtrs<R>& P, const SweepLay<R, DIR>& L, R* sm, int so, int sp, int sa,
+                                     int tid, int nout, R inv_h, bool ok, long long cell0, long long stride) {
   using V = typename PairOf<R>::V;
   constexpr int ST = DIR == 0 ? 1 : kSweepLines;
   const int c = tid % kSweepLines, task = tid / kSweepLines;
@@ -333,10 +332,9 @@ __device__ __forceinline__ void walk(const DevCfg& C, const DevPtrs<R>& P, const
   V dm = v_sub(qc, q1), dp = v_sub(qp, qc);
   V Dm = v_sub(dm, v_sub(q1, q0)), D = v_sub(dp, dm);
   V tm = weno_t<V>(Dm), t = weno_t<V>(D);
-  // the left neighbour's right-face sums (FP32: nl holds the quotients nl/sl;
-  // minmod: the slopes)
+  // the left neighbour's right-face sums (FP32: nl holds the quotients nl/sl)
   V nlp = v_c<V>(0.), slp = v_c<V>(1.);
-  R fm = 0, vm = 0, hprev = 0;  // F, V of the left neighbour; flux at the face before (or its derivative)
+  R fm = 0, hprev = 0;  // F of the left neighbour; flux at the face before (or its derivative)
   R xprev = 0;
   // the value to add to is loaded a cell ahead
   R acc0 = 0;
@@ -349,47 +347,33 @@ __device__ __forceinline__ void walk(const DevCfg& C, const DevPtrs<R>& P, const
     const V dn = v_sub(qn, qp), Dp = v_sub(dn, dp), tp = weno_t<V>(Dp);
     R fc, vc;
     v_split(qc, fc, vc);
-    Face<V> f;
-    if (!MM || !flux) f = weno_face<V>(dm, dp, Dm, D, Dp, tm, t, tp);
+    const Face<V> f = weno_face<V>(dm, dp, Dm, D, Dp, tm, t, tp);
     const R am = *pm;  // of the face left of cell a (a = 2: not used)
     pm += ST;
     if (flux) {
       R h, acc1 = acc0;
       if (!TMA && DIR != 0 && acc && a > 3 && a < nout + 3) acc1 = oa[stride];
-      if constexpr (MM) {
-        // slopes of F and V; 2 H = F + F' + (s - s')/2 - a (V' - V - (s + s')/2)
-        const R th = (R)C.mm_theta;
-        R fa, fb, va, vb, s0, s1, p0, p1;
-        v_split(dm, fa, va);
-        v_split(dp, fb, vb);
-        s0 = mm3<R>(th * fa, (R)0.5 * (fa + fb), th * fb);
-        s1 = mm3<R>(th * va, (R)0.5 * (va + vb), th * vb);
-        v_split(nlp, p0, p1);
-        h = (fm + fc) + (R)0.5 * (p0 - s0) - am * ((vc - vm) - (R)0.5 * (p1 + s1));
-        nlp = v_pair(s0, s1);
+      // 2 H = F_L + F_R - a (V_R - V_L)
+      R n0, n1, m0, m1, r0, r1, corr;
+      v_split(nlp, n0, n1);
+      v_split(f.nr, m0, m1);
+      v_split(f.sr, r0, r1);
+      if constexpr (sizeof(R) == 8) {
+        // one reciprocal for the face's four quotients (the product of the
+        // sums stays far inside double range)
+        R s0, s1;
+        v_split(slp, s0, s1);
+        const R nf = fma(n0, r0, m0 * s0), nv = am * fma(n1, r1, -(m1 * s1)), df = s0 * r0, dv = s1 * r1;
+        corr = fma(nf, dv, nv * df) * fast_rcp(df * dv);
+        nlp = f.nl;
+        slp = f.sl;
       } else {
-        // 2 H = F_L + F_R - a (V_R - V_L)
-        R n0, n1, m0, m1, r0, r1, corr;
-        v_split(nlp, n0, n1);
-        v_split(f.nr, m0, m1);
-        v_split(f.sr, r0, r1);
-        if constexpr (sizeof(R) == 8) {
-          // one reciprocal for the face's four quotients (the product of the
-          // sums stays far inside double range)
-          R s0, s1;
-          v_split(slp, s0, s1);
-          const R nf = fma(n0, r0, m0 * s0), nv = am * fma(n1, r1, -(m1 * s1)), df = s0 * r0, dv = s1 * r1;
-          corr = fma(nf, dv, nv * df) * fast_rcp(df * dv);
-          nlp = f.nl;
-          slp = f.sl;
-        } else {
-          R x0, x1;
-          corr = fma(am, fma(-m1, fast_rcp(r1), n1), fma(m0, fast_rcp(r0), n0));
-          v_split(f.sl, x0, x1);
-          nlp = v_mul(f.nl, v_pair(fast_rcp(x0), fast_rcp(x1)));
-        }
-        h = fma(-sixth, corr, fm + fc);
+        R x0, x1;
+        corr = fma(am, fma(-m1, fast_rcp(r1), n1), fma(m0, fast_rcp(r0), n0));
+        v_split(f.sl, x0, x1);
+        nlp = v_mul(f.nl, v_pair(fast_rcp(x0), fast_rcp(x1)));
       }
+      h = fma(-sixth, corr, fm + fc);
       const R r = kdiv * (h - hprev);
       if (a > 3) {
         *oa = !TMA && DIR != 0 ? acc0 + r : r;
@@ -397,7 +381,6 @@ __device__ __forceinline__ void walk(const DevCfg& C, const DevPtrs<R>& P, const
       }
       hprev = h;
       fm = fc;
-      vm = vc;
     } else {
       if (a > 3) {
         *oa = hprev;
@@ -434,6 +417,97 @@ __device__ __forceinline__ void walk(const DevCfg& C, const DevPtrs<R>& P, const
     tm = t;
     t = tp;
   }
+}
+
+// Generalized minmod: a thread owns F^l and V^l (tasks 0..8) and keeps their
+// slopes, s = mm3(theta dm, (dm + dp)/2, theta dp), with
+// 2 H = F + F' + (s - s')/2 - a (V' - V - (s + s')/2).
+template <class R, int DIR, bool TMA>
+__device__ __forceinline__ void walk_minmod(const DevCfg& C, const DevPtrs<R>& P, const SweepLay<R, DIR>& L, R* sm,
+                                            int so, int sp, int sa, int tid, int nout, R inv_h, bool ok,
+                                            long long cell0, long long stride) {
+  constexpr int ST = DIR == 0 ? 1 : kSweepLines;
+  const int c = tid % kSweepLines, task = tid / kSweepLines;
+  if (task >= 9 || !ok) return;
+  const int vslot = task < 4 ? so + task * L.cells : sp + (task - 4) * L.cells;
+  const bool carried = task >= 4;
+  const bool acc = !TMA && DIR != 0 && !P.res1;
+  R* const line = sm + c * L.ld + ST;
+  const R *pa = line + (task < 4 ? L.offf + task * L.cells : 0), *pb = line + vslot, *pm = line + sa;
+  R* o = DIR == 0 ? line + vslot : P.resd(DIR) + (long long)task * P.stride + cell0 + stride;
+  const R kdiv = (R)-0.5 * inv_h, th = (R)C.mm_theta;
+  R f0, v0, f1, v1, f2, v2;  // cells a - 1, a, a + 1
+  auto load = [&](R& f, R& v) {
+    v = *pb;
+    f = carried ? *pa * v : *pa;
+    pa += ST;
+    pb += ST;
+  };
+  load(f0, v0);
+  load(f1, v1);
+  R sf = 0, sv = 0, hprev = 0;  // slopes of the left neighbour; flux at the face before
+#pragma unroll 3
+  for (int a = 2; a < nout + 4; a++) {
+    load(f2, v2);
+    const R df = f1 - f0, ef = f2 - f1, dv = v1 - v0, ev = v2 - v1;
+    const R tf = mm3<R>(th * df, (R)0.5 * (df + ef), th * ef), tv = mm3<R>(th * dv, (R)0.5 * (dv + ev), th * ev);
+    const R h = (f0 + f1) + (R)0.5 * (sf - tf) - *pm * (dv - (R)0.5 * (sv + tv));
+    pm += ST;
+    if (a > 3) {
+      const R r = kdiv * (h - hprev);
+      *o = acc ? *o + r : r;
+    }
+    o += DIR == 0 ? 1 : stride;
+    hprev = h;
+    sf = tf;
+    sv = tv;
+    f0 = f1;
+    v0 = v1;
+    f1 = f2;
+    v1 = v2;
+  }
+}
+
+// The velocity derivatives of the minmod sweep's cells, (L - R) / h of the
+// WENO5 stencil (genWENOder), a cell a thread: in the walk they would be two
+// tasks of three times the others' length.
+template <class R, int DIR, class Ok, class Base>
+__device__ __forceinline__ void cell_derivatives(const DevPtrs<R>& P, const SweepLay<R, DIR>& L, const R* sm, int tid,
+                                                 int nout, R inv_h, Ok&& line_ok, Base&& cell_of) {
+  using V = typename PairOf<R>::V;
+  constexpr int ST = DIR == 0 ? 1 : kSweepLines;
+  const int lanes = DIR == 0 ? 32 : kSweepLines;  // along x a warp takes a line
+  for (int q = tid / lanes; q < (DIR == 0 ? kSweepLines : nout); q += kSweepThreads / lanes)
+    for (int r = tid % lanes; r < (DIR == 0 ? nout : kSweepLines); r += lanes) {
+      const int c = DIR == 0 ? q : r, a = NG + (DIR == 0 ? r : q);
+      if (!line_ok(c)) continue;
+      const R* s = sm + c * L.ld + a * ST;
+      const long long g = cell_of(c, a);
+#pragma unroll
+      for (int l = 0; l < 4; l += 2) {
+        V x[5], d[4], D[3], t[3];
+#pragma unroll
+        for (int m = 0; m < 5; m++) x[m] = v_pair(s[(1 + l) * L.cells + (m - 2) * ST], s[(2 + l) * L.cells + (m - 2) * ST]);
+#pragma unroll
+        for (int m = 0; m < 4; m++) d[m] = v_sub(x[m + 1], x[m]);
+#pragma unroll
+        for (int m = 0; m < 3; m++) {
+          D[m] = v_sub(d[m + 1], d[m]);
+          t[m] = weno_t<V>(D[m]);
+        }
+        const Face<V> f = weno_face<V>(d[1], d[2], D[0], D[1], D[2], t[0], t[1], t[2]);
+        R n[2], sl[2], m0[2], sr[2], gsum[2];
+        v_split(f.nl, n[0], n[1]);
+        v_split(f.sl, sl[0], sl[1]);
+        v_split(f.nr, m0[0], m0[1]);
+        v_split(f.sr, sr[0], sr[1]);
+        v_split(v_add(d[1], d[2]), gsum[0], gsum[1]);
+#pragma unroll
+        for (int k = 0; k < 2; k++)
+          P.du((l + k) * 3 + DIR)[g] =
+              inv_h * fma((R)(-1. / 6.), n[k] * fast_rcp(sl[k]) - m0[k] * fast_rcp(sr[k]), (R)0.5 * gsum[k]);
+      }
+    }
 }
 
 // --------------------------------------------------------------- the tile
@@ -544,8 +618,15 @@ __device__ __forceinline__ void sweep_tile(const DevCfg& C, const DevPtrs<R>& P,
   __syncthreads();
 
   // ---- the walk along the lines
-  walk<R, DIR, MM, TMA>(C, P, L, sm, so, sp, sa, tid, nout, inv_h, line_ok(tid % kSweepLines),
-                        line_base(tid % kSweepLines) + (long long)a0 * stride, stride);
+  const bool ok = line_ok(tid % kSweepLines);
+  const long long cell0 = line_base(tid % kSweepLines) + (long long)a0 * stride;
+  if constexpr (MM) {
+    cell_derivatives<R, DIR>(P, L, sm, tid, nout, inv_h, line_ok,
+                             [&](int c, int a) { return line_base(c) + (long long)(a0 + a) * stride; });
+    walk_minmod<R, DIR, TMA>(C, P, L, sm, so, sp, sa, tid, nout, inv_h, ok, cell0, stride);
+  } else {
+    walk<R, DIR, TMA>(P, L, sm, so, sp, sa, tid, nout, inv_h, ok, cell0, stride);
+  }
   if constexpr (DIR == 0) {
     // a warp's lanes walked along rows a pitch apart: the results, left in
     // the tile, go out row by row
@@ -558,8 +639,10 @@ __device__ __forceinline__ void sweep_tile(const DevCfg& C, const DevPtrs<R>& P,
       for (int a = NG + tid % 32; a < NG + nout; a += 32) {
 #pragma unroll
         for (int q = 0; q < 9; q++) r0[(long long)q * P.stride + a] = s[(q < 4 ? so + q * L.cells : sp + (q - 4) * L.cells) + a];
+        if (!MM) {
 #pragma unroll
-        for (int q = 0; q < 4; q++) d0[(long long)(q * 3) * P.stride + a] = s[(1 + q) * L.cells + a];
+          for (int q = 0; q < 4; q++) d0[(long long)(q * 3) * P.stride + a] = s[(1 + q) * L.cells + a];
+        }
       }
     }
   }
