@@ -361,14 +361,14 @@ def algorithmic_bytes(cfg, kernel: str) -> float:
     it has to read and write once; halo re-reads not counted)."""
     w = 4 if cfg.precision == 1 else 8
     if kernel.startswith("k_dir"):
-        # reads e, u(4), T(4), pi(5); writes (or read+writes) res(9) and du(4)
-        first = kernel.endswith("x")
-        return w * (14 + (9 if first else 18) + 4)
+        # reads e, u(4), T(4), pi(5); writes the direction's res(9) and du(4)
+        return w * (14 + 9 + 4)
+    dirs = 2 if cfg.boost_invariant else 3  # sets of res and du
     if kernel == "k_update_stage1":
-        # reads res 9, du 12, e, u 4, pu 4, A 9; writes B 9, v1t 4, e, u 4, pu 4
-        return w * (9 + 12 + 1 + 4 + 4 + 9 + 9 + 4 + 1 + 4 + 4)
-    # stage 2: reads res 9, du 12, e, u 4, pu 4, B 9, A 4, v1t 4; writes A 9, e, u 4
-    return w * (9 + 12 + 1 + 4 + 4 + 9 + 4 + 4 + 9 + 1 + 4)
+        # reads res, du, e, u 4, pu 4, A 9; writes B 9, v1t 4, e, u 4, pu 4
+        return w * (13 * dirs + 1 + 4 + 4 + 9 + 9 + 4 + 1 + 4 + 4)
+    # stage 2: reads res, du, e, u 4, pu 4, B 9, A 9, v1t 4; writes A 9, e, u 4
+    return w * (13 * dirs + 1 + 4 + 4 + 9 + 9 + 4 + 9 + 1 + 4)
 
 
 # DRAM bytes (read + write) per interior cell and launch, from one ncu capture
@@ -376,22 +376,22 @@ def algorithmic_bytes(cfg, kernel: str) -> float:
 # sweeps, profiles/update_kernel_*.md for the updates), scaled to a full launch
 # by the cells processed
 MEASURED_TRAFFIC_PER_CELL = {
-    ("fp64", "k_dir_x"): 153.0, ("fp64", "k_dir_y"): 230.0, ("fp64", "k_dir_eta"): 258.0,
-    ("fp64", "k_update_stage1"): 469.0, ("fp64", "k_update_stage2"): 500.0,
-    ("mixed", "k_dir_x"): 65.0, ("mixed", "k_dir_y"): 104.0, ("mixed", "k_dir_eta"): 114.0,
-    ("mixed", "k_update_stage1"): 192.0, ("mixed", "k_update_stage2"): 226.0,
+    ("fp64", "k_dir_x"): 136.0, ("fp64", "k_dir_y"): 154.0, ("fp64", "k_dir_eta"): 180.0,
+    ("fp64", "k_update_stage1"): 634.0, ("fp64", "k_update_stage2"): 669.0,
+    ("mixed", "k_dir_x"): 66.0, ("mixed", "k_dir_y"): 66.0, ("mixed", "k_dir_eta"): 75.0,
+    ("mixed", "k_update_stage1"): 293.0, ("mixed", "k_update_stage2"): 320.0,
 }
 
 
 # the bound that does hold for the step kernels: the share of peak of the
 # pipe or issue rate that limits each, from the same ncu captures
 MEASURED_COMPUTE_BOUND = {
-    ("fp64", "k_dir_x"): ("fp64 pipe", 0.753), ("fp64", "k_dir_y"): ("fp64 pipe", 0.724),
-    ("fp64", "k_dir_eta"): ("fp64 pipe", 0.756), ("fp64", "k_update_stage1"): ("fp64 pipe", 0.323),
-    ("fp64", "k_update_stage2"): ("fp64 pipe", 0.347),
-    ("mixed", "k_dir_x"): ("fma pipe", 0.680), ("mixed", "k_dir_y"): ("fma pipe", 0.650),
-    ("mixed", "k_dir_eta"): ("fma pipe", 0.693), ("mixed", "k_update_stage1"): ("issue", 0.503),
-    ("mixed", "k_update_stage2"): ("issue", 0.507),
+    ("fp64", "k_dir_x"): ("fp64 pipe", 0.544), ("fp64", "k_dir_y"): ("fp64 pipe", 0.557),
+    ("fp64", "k_dir_eta"): ("fp64 pipe", 0.566), ("fp64", "k_update_stage1"): ("issue", 0.352),
+    ("fp64", "k_update_stage2"): ("issue", 0.364),
+    ("mixed", "k_dir_x"): ("issue", 0.588), ("mixed", "k_dir_y"): ("issue", 0.579),
+    ("mixed", "k_dir_eta"): ("issue", 0.641), ("mixed", "k_update_stage1"): ("issue", 0.447),
+    ("mixed", "k_update_stage2"): ("issue", 0.450),
 }
 
 
@@ -459,7 +459,7 @@ def run_ours(args, rank, world, dist):
     H = C.make_hydro(cfg, inp)
     A.check(A.lib().vh_set_stream(H.h, ctypes_void_p(stream.cuda_stream)), H.h)
     cells = cfg.nx * cfg.ny * (1 if cfg.boost_invariant else cfg.nz)
-    launches_per_step = 2 * ((2 if cfg.boost_invariant else 3) + 1)
+    launches_per_step = 4  # per stage: the sweeps of every direction, the update
 
     H.step(args.warmup)
     torch.cuda.synchronize()
@@ -664,7 +664,7 @@ def mixed_record(args, fp64_ms_per_step: float) -> dict:
             "dtype": "f32 state, fluxes, reconstruction, sources / f64 root-find, EOS inversion, conservation sums",
             "errors_vs_fp64": errs, "fp64_perturbed_1e-7_vs_fp64": base, "error_steps": marks,
             "error_tau_end_fm": tau_end, "error_norms": ERROR_NORMS, "clocks": clocks,
-            "gpu_launches": 2 * ((2 if cfg32.boost_invariant else 3) + 1) * args.steps,
+            "gpu_launches": 4 * args.steps,
             "roofline": roofline(cfg32, "mixed", cells, per_launch, share, top),
             "config": dict(desc, workload=args.workload + " (precision form)")}
 
