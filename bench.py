@@ -162,6 +162,15 @@ def _ref_window_worker(args):
     return out
 
 
+def reference_missing(workload: str) -> str | None:
+    """why the reference's CPU step of `workload` cannot run here (its build
+    needs the reference's headers), or None"""
+    name = f"libref_{'window_lbi' if workload == 'ensemble' else 'window_3d'}.so"
+    if os.path.exists(os.path.join(ROOT, "oracle", "_ref", name)):
+        return None
+    return f"oracle/_ref/{name} is not built (make -C oracle needs the reference's NEWEST5 headers)"
+
+
 def reference_windows(workload: str, seconds: float, n_samples: int, procs: int):
     """Aggregate cell-updates/s of the reference's CPU step over `procs` host
     processes on windows of a Glauber state of `workload` (the benchmarked
@@ -822,7 +831,10 @@ def ensemble_record(args) -> dict:
                       "b_fm": [0, 12], "seeds": [0, n - 1], "dtau_fm": ENS_DTAU, "tau0_fm": ENS_TAU0,
                       "tau_max_fm": ENS_TAU_MAX, "t_freeze_gev": ENS_T_FO, "floor_gev_fm3": floor,
                       "eos": "synthetic table (2000 rows)", "eta_over_s": 0.08}}
-    if args.cpu_seconds > 0:
+    if args.cpu_seconds > 0 and reference_missing("ensemble"):
+        out["cpu_baseline"] = {"value": None, "unit": "events/s", "kind": "reference",
+                               "unavailable": reference_missing("ensemble")}
+    elif args.cpu_seconds > 0:
         rates, procs, desc = reference_windows("ensemble", args.cpu_seconds, 1, reference_procs())
         cpu_seconds_total = mixed["cell_updates"] / rates[0]
         out["cpu_baseline"] = {"value": mixed["completed"] / cpu_seconds_total, "unit": "events/s", "cores": procs,
@@ -1066,6 +1078,9 @@ def ctypes_void_p(v):
 def reference_arm(args, world):
     """the reference's CPU step on the benchmarked workload (windows of its
     Glauber state, all host cores); rank 0 only"""
+    if reference_missing(args.workload):
+        print(json.dumps({"impl": "reference", "unavailable": reference_missing(args.workload)}), flush=True)
+        return
     t0 = time.perf_counter()
     procs = reference_procs()
     rates, procs, desc = reference_windows(args.workload, args.ref_sample_seconds, args.warmup + args.steps, procs)
@@ -1118,7 +1133,10 @@ def main():
             out["ensemble"] = ensemble_record(args)
         if "adjoint" in subs:
             out["adjoint"] = adjoint_record(args)
-        if args.cpu_seconds > 0:
+        if args.cpu_seconds > 0 and reference_missing(args.workload):
+            out["cpu_baseline"] = {"value": None, "unit": METRIC, "kind": "reference",
+                                   "unavailable": reference_missing(args.workload)}
+        elif args.cpu_seconds > 0:
             rates, procs, desc = reference_windows(args.workload, args.cpu_seconds, 1, reference_procs())
             out["cpu_baseline"] = {"value": rates[0], "unit": METRIC, "cores": procs, "kind": "reference",
                                    "sample": f"{desc}; {args.cpu_seconds:.0f} s; {cpu_model()}"}
