@@ -114,62 +114,73 @@ __global__ void __launch_bounds__(kThreads) k_fo_emit(vh_fo::Geo g, const double
 }
 
 // ---- spectra
-// A block sums a share of the elements for kBins momentum bins at once, one
-// element a thread at a time: what depends on the element alone (in 3+1D
-// cosh and sinh of y - eta; in 2+1D the Bessel functions, which depend on the
-// bin through m_T only) is formed once for all of them, and the bins'
-// exponentials are independent of one another.  One block per bin had formed
-// them per bin, with 128 blocks on the GPU (0.8 M elements, 8 x 16 bins:
-// 4.06 ms; now 0.78, bound by the FP64 exponentials).  bins: m_T, p_x, p_y, kBins a tile, zeros where a tile has fewer;
-// part: a partial sum per bin and share of the elements.
-constexpr int kBins = 16, kCfThreads = 128;
+// A block sums a share of the elements for kBins momentum bins at once, 128
+// elements at a time: the block copies their rows into shared memory, a thread
+// forms what depends on its element alone (in 3+1D cosh and sinh of y - eta;
+// in 2+1D the Bessel functions, which depend on the bin through m_T only),
+// then each warp takes kWarpBins bins, held in registers, through all 128.
+// 0.8 M elements and 8 x 16 bins: 0.33 ms, bound by the FP64 exponentials.  An
+// element a thread with all 16 bins held 128 registers with spills and read its
+// row 96 bytes from the next lane's, 0.79 ms; one block per bin before that,
+// forming the element's part anew for each, 4.06 ms.  4 blocks per SM (102
+// registers): with 5, 6 and 8 the call takes 0.93, 0.82 and 0.86 ms against 0.76.
+// bins: m_T, p_x, p_y, kBins a tile, zeros where a tile has fewer; part: a
+// partial sum per bin and share of the elements.
+constexpr int kBins = 16, kCfThreads = 128, kCfWarps = kCfThreads / 32, kWarpBins = kBins / kCfWarps;
 template <int D>
 __global__ void __launch_bounds__(kCfThreads, 4) k_cooper_frye(const double* __restrict__ el, long long count,
                                                              const double* __restrict__ bins, double y, double t_fo,
                                                              double* __restrict__ part) {
-  __shared__ double bin[kBins][3], red[kCfThreads / 32][kBins];
-  const int tid = threadIdx.x;
-  if (tid < 3 * kBins) bin[tid / 3][tid % 3] = bins[(long long)blockIdx.x * 3 * kBins + tid];
-  __syncthreads();
-  const double it = 1.0 / t_fo;
-  double acc[kBins];
+  // a row's words; an odd pitch keeps lanes an element apart on their own banks
+  constexpr int W = D == 3 ? vh_fo::kW2 : vh_fo::kW3, P = W | 1;
+  __shared__ double row[kCfThreads * P], term[6][kCfThreads];
+  const int tid = threadIdx.x, lane = tid & 31;
+  const double* mine = bins + ((long long)blockIdx.x * kBins + tid / 32 * kWarpBins) * 3;
+  double mt[kWarpBins], px[kWarpBins], py[kWarpBins], acc[kWarpBins];
 #pragma unroll
-  for (int b = 0; b < kBins; b++) acc[b] = 0;
-  for (long long e = (long long)blockIdx.y * kCfThreads + tid; e < count; e += (long long)gridDim.y * kCfThreads) {
-    if constexpr (D == 4) {
-      const double* q = el + vh_fo::kW3 * e;
-      const double tau = q[0], ch = cosh(y - q[3]), sh = sinh(y - q[3]);
-      // p.dSigma = m_T A + p_x B + p_y C, p.u / T = m_T U - p_x V - p_y W
-      const double A = ch * q[4] + sh / tau * q[7], B = q[5], C = q[6];
-      const double U = (ch * q[8] - tau * sh * q[11]) * it, V = q[9] * it, W = q[10] * it;
-#pragma unroll
-      for (int b = 0; b < kBins; b++) {
-        const double mt = bin[b][0], px = bin[b][1], py = bin[b][2];
-        acc[b] += (mt * A + px * B + py * C) * exp(px * V + py * W - mt * U);
+  for (int b = 0; b < kWarpBins; b++) {
+    mt[b] = D == 3 ? 1.0 : mine[3 * b];  // 2+1D: within the element's part
+    px[b] = mine[3 * b + 1];
+    py[b] = mine[3 * b + 2];
+    acc[b] = 0;
+  }
+  const double it = 1.0 / t_fo, mt_tile = bins[(long long)blockIdx.x * kBins * 3];
+  for (long long e0 = (long long)blockIdx.y * kCfThreads; e0 < count; e0 += (long long)gridDim.y * kCfThreads) {
+    const int live = (int)(count - e0 < kCfThreads ? count - e0 : kCfThreads);
+    // row was last read before the previous turn's second barrier
+    for (int w = tid; w < live * W; w += kCfThreads) row[w / W * P + w % W] = el[e0 * W + w];
+    __syncthreads();
+    // the term of a bin: (m_T A + p_x B + p_y C) exp(p_x V + p_y Y - m_T U)
+    double A = 0, B = 0, C = 0, U = 0, V = 0, Y = 0;
+    if (tid < live) {
+      const double* q = row + tid * P;
+      if constexpr (D == 4) {
+        const double tau = q[0], ch = cosh(y - q[3]), sh = sinh(y - q[3]);
+        A = ch * q[4] + sh / tau * q[7], B = q[5], C = q[6];
+        U = (ch * q[8] - tau * sh * q[11]) * it, V = q[9] * it, Y = q[10] * it;
+      } else {
+        double k0e, k1e;
+        U = mt_tile * q[6] * it;
+        vh_fo::bessel_k01e(U, &k0e, &k1e);
+        A = 2 * mt_tile * k1e * q[3], B = 2 * k0e * q[4], C = 2 * k0e * q[5], V = q[7] * it, Y = q[8] * it;
       }
-    } else {
-      const double* q = el + vh_fo::kW2 * e;
-      const double mt = bin[0][0], a = mt * q[6] * it;
-      double k0e, k1e;
-      vh_fo::bessel_k01e(a, &k0e, &k1e);
-      const double A = 2 * mt * k1e * q[3], B = 2 * k0e * q[4], C = 2 * k0e * q[5], V = q[7] * it, W = q[8] * it;
+    }
+    term[0][tid] = A, term[1][tid] = B, term[2][tid] = C;
+    term[3][tid] = U, term[4][tid] = V, term[5][tid] = Y;
+    __syncthreads();
+#pragma unroll 1
+    for (int i = lane; i < live; i += 32) {
+      const double a = term[0][i], b1 = term[1][i], c = term[2][i], u = term[3][i], v = term[4][i], yy = term[5][i];
 #pragma unroll
-      for (int b = 0; b < kBins; b++) {
-        const double px = bin[b][1], py = bin[b][2];
-        acc[b] += (A + px * B + py * C) * exp(px * V + py * W - a);
-      }
+      for (int b = 0; b < kWarpBins; b++)
+        acc[b] += (mt[b] * a + px[b] * b1 + py[b] * c) * exp(px[b] * v + py[b] * yy - mt[b] * u);
     }
   }
 #pragma unroll
-  for (int b = 0; b < kBins; b++) {
+  for (int b = 0; b < kWarpBins; b++) {
     for (int o = 16; o > 0; o >>= 1) acc[b] += __shfl_down_sync(0xffffffffu, acc[b], o);
-    if ((tid & 31) == 0) red[tid >> 5][b] = acc[b];
-  }
-  __syncthreads();
-  if (tid < kBins) {
-    double s = 0;
-    for (int w = 0; w < kCfThreads / 32; w++) s += red[w][tid];
-    part[((long long)blockIdx.x * kBins + tid) * gridDim.y + blockIdx.y] = s;
+    if (lane == 0)
+      part[((long long)blockIdx.x * kBins + tid / 32 * kWarpBins + b) * gridDim.y + blockIdx.y] = acc[b];
   }
 }
 // the shares' sums, one warp per slot; slot q of tile t is the bin
