@@ -42,6 +42,7 @@ struct Tables {
   int* steps;
   unsigned long long* tmax_bits;
   unsigned int* flag;      // per-event failure bits (the event's DevPtrs status)
+  unsigned int* failed;    // the same as of the phase before
   const int4* items;       // flux tiles: {event, tile along, tile across, cells of a tile + 256 direction}
   int n_first, n_items;    // tiles up to n_first, then (behind a barrier) the others
   const int2* uitems;      // {event, chunk of blockDim cells}
@@ -72,7 +73,9 @@ __device__ inline DevCfg event_cfg(const DevCfg& C0, int nx, int ny) {
 
 // Grid-wide barrier among the co-resident blocks of a cooperative launch.
 // The wait is bounded: after ~2 s the block sets the timeout flag and
-// returns false, and every block leaves the kernel at its next check.
+// returns false, and every block leaves the kernel at its next check.  Other
+// blocks write that flag: one thread reads it for the block, so that a block
+// leaves as a whole.
 __device__ inline bool grid_barrier(unsigned int* bar, long long max_spins = 1ll << 24) {
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -92,8 +95,7 @@ __device__ inline bool grid_barrier(unsigned int* bar, long long max_spins = 1ll
     }
     __threadfence();
   }
-  __syncthreads();
-  return *(volatile unsigned int*)(bar + 2) == 0;
+  return !__syncthreads_or(threadIdx.x == 0 && *(volatile unsigned int*)(bar + 2) != 0);
 }
 
 // one tile of an event's flux sweep along DIR
@@ -115,6 +117,9 @@ __global__ void __launch_bounds__(kSweepThreads, MINB) k_batch(Args<R> A, int ns
   __shared__ double red[32];
   for (int s = 0; s < nsteps; s++) {
     for (int stage = 0; stage < 2; stage++) {
+      // the flags the update goes by; no sweep through the cache raises one
+      if (blockIdx.x == 0)
+        for (int ev = threadIdx.x; ev < T.n_events; ev += blockDim.x) T.failed[ev] = T.flag[ev];
       // ---- flux sweeps: all tiles at once where the pool has a divergence
       // set per direction, else the x tiles and, behind a barrier, the y
       // tiles that add to them
@@ -137,12 +142,15 @@ __global__ void __launch_bounds__(kSweepThreads, MINB) k_batch(Args<R> A, int ns
         }
         if (!grid_barrier(T.bar)) return;
       }
-      // ---- update: sources, RK, root-find, ghosts; stage 2 also reduces max T
+      // ---- update: sources, RK, root-find, ghosts; stage 2 also reduces max T.
+      // Other blocks' root-finds raise flags during this phase, and warps that
+      // read a flag at different times would part at the barriers in the loop:
+      // `failed` holds the flags as they were before it.
       unsigned long long my_it = 0;
       for (int it = blockIdx.x; it < T.n_u; it += gridDim.x) {
         const int2 w = T.uitems[it];
         const int ev = w.x;
-        if (T.state[ev] != EV_RUNNING || T.flag[ev]) continue;
+        if (T.state[ev] != EV_RUNNING || T.failed[ev]) continue;
         const DevCfg C = event_cfg(A.C0, T.nx[ev], T.ny[ev]);
         DevPtrs<R> P = A.pool.shifted(T.off[ev]);
         P.status = T.flag + ev;
@@ -243,7 +251,7 @@ struct vh_batch {
   int *d_nx = nullptr, *d_ny = nullptr, *d_state = nullptr, *d_steps = nullptr, *d_running = nullptr;
   double *d_tau = nullptr, *d_dtau = nullptr, *d_taumax = nullptr;
   unsigned long long *d_tmax = nullptr, *d_iters = nullptr;
-  unsigned int *d_flag = nullptr, *d_bar = nullptr;
+  unsigned int *d_flag = nullptr, *d_bar = nullptr;  // flags and, behind them, their copies
   int4* d_items = nullptr;
   int n_first = 0, n_items = 0;
   int arrays = 0;  // of the pool: 52, or 61 with a divergence set for y
@@ -387,7 +395,7 @@ extern "C" int vh_batch_create(const vh_config* cfg, int n_events, const int* nx
       !ok(cudaMalloc(&b->d_tau, sizeof(double) * n)) || !ok(cudaMalloc(&b->d_dtau, sizeof(double) * n)) ||
       !ok(cudaMalloc(&b->d_taumax, sizeof(double) * n)) ||
       !ok(cudaMalloc(&b->d_tmax, sizeof(unsigned long long) * n)) ||
-      !ok(cudaMalloc(&b->d_iters, sizeof(unsigned long long))) || !ok(cudaMalloc(&b->d_flag, sizeof(unsigned int) * n)) ||
+      !ok(cudaMalloc(&b->d_iters, sizeof(unsigned long long))) || !ok(cudaMalloc(&b->d_flag, 2 * sizeof(unsigned int) * n)) ||
       !ok(cudaMalloc(&b->d_bar, sizeof(unsigned int) * 4)) || !ok(cudaMalloc(&b->stage, sizeof(double) * 18 * big)))
     return fail("tables");
   if (!ok(cudaMemcpy(b->d_off, b->off.data(), sizeof(long long) * n, cudaMemcpyHostToDevice)) ||
@@ -411,7 +419,7 @@ extern "C" int vh_batch_reset(vh_batch* b) {
   VB_CUDA(b, cudaMemcpy(b->d_state, zeros.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
   VB_CUDA(b, cudaMemcpy(b->d_steps, zeros.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
   VB_CUDA(b, cudaMemset(b->d_tmax, 0, sizeof(unsigned long long) * n));
-  VB_CUDA(b, cudaMemset(b->d_flag, 0, sizeof(unsigned int) * n));
+  VB_CUDA(b, cudaMemset(b->d_flag, 0, 2 * sizeof(unsigned int) * n));
   VB_CUDA(b, cudaMemset(b->d_bar, 0, sizeof(unsigned int) * 4));
   VB_CUDA(b, cudaMemset(b->d_iters, 0, sizeof(unsigned long long)));
   VB_CUDA(b, cudaMemcpy(b->d_running, &n, sizeof(int), cudaMemcpyHostToDevice));
@@ -540,7 +548,7 @@ static int launch_variant(vh_batch* b, cudaStream_t s, int nsteps, bool query_on
   A.pool = pool_ptrs<R>(b);
   Tables& T = A.T;
   T.n_events = b->n; T.off = b->d_off; T.nx = b->d_nx; T.ny = b->d_ny; T.tau = b->d_tau; T.dtau = b->d_dtau;
-  T.tau_max = b->d_taumax; T.state = b->d_state; T.steps = b->d_steps; T.tmax_bits = b->d_tmax; T.flag = b->d_flag;
+  T.tau_max = b->d_taumax; T.state = b->d_state; T.steps = b->d_steps; T.tmax_bits = b->d_tmax; T.flag = b->d_flag; T.failed = b->d_flag + b->n;
   T.items = b->d_items; T.n_first = b->n_first; T.n_items = b->n_items;
   T.uitems = b->d_u; T.n_u = b->n_ui; T.bar = b->d_bar; T.running = b->d_running; T.iters = b->d_iters;
   T.t_freeze_gev = b->t_freeze_gev;
