@@ -306,7 +306,10 @@ int vh_step_static(const vh_config* cfg, double* state, const double* eos_dev, d
  * breaks, NEWEST5/main.cpp:188-205, applied per event), or fails alone
  * (root-find / causality) while the others continue.  The common physics
  * (EOS, transport, precision, reconstruction, dx, dy) comes from cfg; its
- * grid and time fields are ignored. */
+ * grid and time fields are ignored.  The pool takes 61 arrays of a cell's
+ * state and scratch where that is no more than a quarter of the free device
+ * memory at vh_batch_create, else (or with VH_BATCH_SETS=1 in the
+ * environment) 52, with one more barrier a stage. */
 typedef struct vh_batch vh_batch;
 enum { VH_EVENT_RUNNING = 0, VH_EVENT_FROZEN = 1, VH_EVENT_TAUMAX = 2, VH_EVENT_FAILED = 3 };
 int vh_batch_create(const vh_config* cfg, int n_events, const int* nx, const int* ny, const double* tau0,

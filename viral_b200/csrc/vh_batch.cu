@@ -12,6 +12,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <fstream>
 #include <sstream>
@@ -352,13 +353,16 @@ extern "C" int vh_batch_create(const vh_config* cfg, int n_events, const int* nx
   C.etas0 = cfg->etas0; C.etas1 = cfg->etas1; C.etas_tc = cfg->etas_tc; C.hbarc = cfg->hbarc;
   C.taupi_kind = cfg->taupi_kind; C.taupi_c = cfg->taupi_const; C.cold = cfg->cold_plasma != 0;
   C.mm_theta = cfg->minmod_theta;
+  cudaError_t last = cudaSuccess;
   auto fail = [&](const char* what) {
     g_batch_err = std::string("vh_batch_create: ") + what + ": " + b->err;
     vh_batch_destroy(b);
-    return VH_E_CUDA;
+    cudaGetLastError();
+    return last == cudaErrorMemoryAllocation ? VH_E_NOMEM : VH_E_CUDA;
   };
   // a CUDA call's success, recording its error for fail()
   auto ok = [&](cudaError_t ce) {
+    last = ce;
     if (ce != cudaSuccess) b->err = cudaGetErrorString(ce);
     return ce == cudaSuccess;
   };
@@ -376,18 +380,6 @@ extern "C" int vh_batch_create(const vh_config* cfg, int n_events, const int* nx
     C.eos_d = b->eos_d; C.eos_f = b->eos_f;
   }
   b->cfg.eos_e = b->cfg.eos_p = b->cfg.eos_cs2 = b->cfg.eos_t = nullptr;
-  // 52 arrays an event, and nine more for the y sweeps' divergence where
-  // they fit
-  b->arrays = kPoolArrays + 9;
-  cudaError_t ce = cudaMalloc(&b->pool, (size_t)b->arrays * tot * b->esz);
-  if (ce == cudaErrorMemoryAllocation) {
-    cudaGetLastError();
-    b->arrays = kPoolArrays;
-    ce = cudaMalloc(&b->pool, (size_t)b->arrays * tot * b->esz);
-  }
-  const size_t pool_bytes = (size_t)b->arrays * tot * b->esz;
-  if (ce != cudaSuccess) { b->err = cudaGetErrorString(ce); g_batch_err = "vh_batch_create: pool: " + b->err; vh_batch_destroy(b); return VH_E_NOMEM; }
-  if (!ok(cudaMemset(b->pool, 0, pool_bytes))) return fail("pool");
   const int n = n_events;
   if (!ok(cudaMalloc(&b->d_off, sizeof(long long) * n)) || !ok(cudaMalloc(&b->d_nx, sizeof(int) * n)) ||
       !ok(cudaMalloc(&b->d_ny, sizeof(int) * n)) || !ok(cudaMalloc(&b->d_state, sizeof(int) * n)) ||
@@ -404,6 +396,17 @@ extern "C" int vh_batch_create(const vh_config* cfg, int n_events, const int* nx
       !ok(cudaMemcpy(b->d_dtau, b->dtau.data(), sizeof(double) * n, cudaMemcpyHostToDevice)) ||
       !ok(cudaMemcpy(b->d_taumax, b->tau_max.data(), sizeof(double) * n, cudaMemcpyHostToDevice)))
     return fail("tables");
+  // The pool last, when all else has its memory: 52 arrays an event, and nine
+  // more for the y sweeps' divergence, which spare the barrier between the x
+  // and the y tiles, where that takes no more than a quarter of what is free
+  // (VH_BATCH_SETS=1 in the environment: never).  A larger ensemble leaves a
+  // caller what it always left.
+  size_t avail = 0, total = 0;
+  if (!ok(cudaMemGetInfo(&avail, &total))) return fail("memory");
+  const char* sets = std::getenv("VH_BATCH_SETS");
+  const size_t one = (size_t)tot * b->esz;
+  b->arrays = (kPoolArrays + 9) * one <= avail / 4 && !(sets && !std::strcmp(sets, "1")) ? kPoolArrays + 9 : kPoolArrays;
+  if (!ok(cudaMalloc(&b->pool, b->arrays * one)) || !ok(cudaMemset(b->pool, 0, b->arrays * one))) return fail("pool");
   b->t_freeze_gev = t_freeze_gev;
   if (vh_batch_reset(b) != VH_OK) return fail("reset");
   if (build_items(b) != VH_OK) return fail("items");
