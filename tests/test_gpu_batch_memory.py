@@ -77,3 +77,24 @@ def test_what_fits_with_52_arrays_is_created():
             B.init_event(0, e, 0 * e, 0 * e)
             B.run(1)
             assert B.events()[2][0] == EVENT_RUNNING
+
+
+def test_tuning_needs_room_for_the_state_alone():
+    """a pool of 61 arrays and 40 arrays' memory left: the trials' copy is of
+    18, and the states are as before"""
+    cfg = C.glauber_config(nx=8, ny=8, boost_invariant=True)
+    sides = [500] * 20
+    array = 8 * sum((s + 6) ** 2 for s in sides)
+    with Batch(cfg, sides, tau0=cfg.tau0, dtau=cfg.dtau, tau_max=100.0, t_freeze_gev=0.0) as B:
+        c = C.glauber_config(nx=500, ny=500, boost_invariant=True)
+        inp = C.glauber_inputs(c, b=4.0, seed=1)
+        for ev in range(len(sides)):
+            B.init_event(ev, inp["e"] * (1 + 0.01 * ev), inp["ux"], inp["uy"])
+        before = [B.event_state(ev) for ev in (0, 19)]
+        B.run(1)  # allocates what a run needs
+        B.init_event(0, inp["e"], inp["ux"], inp["uy"])
+        B.init_event(19, inp["e"] * 1.19, inp["ux"], inp["uy"])
+        with Tight(40 * array):
+            assert B.autotune(None, probe_steps=1) > 0
+        for ev, want in zip((0, 19), before):
+            assert np.array_equal(B.event_state(ev), want)

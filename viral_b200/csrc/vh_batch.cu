@@ -729,20 +729,21 @@ extern "C" int vh_batch_autotune(vh_batch* b, const char* cache_path, int probe_
       }
     }
   }
-  // save the state the trials will advance
-  const size_t pool_bytes = (size_t)b->arrays * b->ntot * b->esz;
+  // save the state the trials will advance: the pool's first 18 arrays (the
+  // others are written before they are read in every step)
+  const size_t saved = (size_t)18 * b->ntot * b->esz;
   void* save = nullptr;
-  VB_CUDA(b, cudaMalloc(&save, pool_bytes));
-  // put the saved pool back; on failure free the copy and report
+  VB_CUDA(b, cudaMalloc(&save, saved));
+  // put the state back; on failure free the copy and report
   auto restore = [&]() {
-    const cudaError_t e = cudaMemcpy(b->pool, save, pool_bytes, cudaMemcpyDeviceToDevice);
+    const cudaError_t e = cudaMemcpy(b->pool, save, saved, cudaMemcpyDeviceToDevice);
     if (e != cudaSuccess) {
       b->err = std::string("vh_batch_autotune: restoring the pool: ") + cudaGetErrorString(e);
       cudaFree(save);
     }
     return e == cudaSuccess;
   };
-  if (const cudaError_t e = cudaMemcpy(save, b->pool, pool_bytes, cudaMemcpyDeviceToDevice); e != cudaSuccess) {
+  if (const cudaError_t e = cudaMemcpy(save, b->pool, saved, cudaMemcpyDeviceToDevice); e != cudaSuccess) {
     b->err = std::string("vh_batch_autotune: saving the pool: ") + cudaGetErrorString(e);
     cudaFree(save);
     return VH_E_CUDA;
