@@ -333,10 +333,11 @@ int vh_batch_run(vh_batch* b, int max_steps, double* seconds, int* graph_used);
 int vh_batch_events(vh_batch* b, double* tau, int* steps, int* state);
 /* one event's 18 canonical fields (doubles, its ghost-inclusive grid) */
 int vh_batch_get_event_state(vh_batch* b, int ev, double* host18);
-/* pick the persistent kernel's tile shape (lines per tile), occupancy,
- * flux-loop unroll and steps per launch by timing probe_steps steps of each
- * candidate; cached by device, precision and event-size histogram in
- * cache_path (NULL: no cache) */
+/* pick the persistent kernel's occupancy (blocks per SM) and steps per launch
+ * by timing probe_steps steps of each candidate; cached by device, precision,
+ * event-size histogram, reconstruction, pool layout and the candidates
+ * themselves in cache_path (NULL: no cache).  Tiles have 8 lines and the flux
+ * loop one form: lines_per_tile is 8 and unroll 1 for every variant. */
 int vh_batch_autotune(vh_batch* b, const char* cache_path, int probe_steps, double* best_ms_per_step);
 int vh_batch_set_tuning(vh_batch* b, int variant, int steps_per_launch, int use_graph);
 int vh_batch_get_tuning(vh_batch* b, int* variant, int* steps_per_launch, int* lines_per_tile, int* blocks_per_sm,

@@ -4,8 +4,8 @@
 // grid-wide barriers between the phases.  Each event has its own tau, dtau
 // and stopping rule (maximum temperature below t_freeze, or tau_max), the
 // reference's main-loop break (NEWEST5/main.cpp:188-205) applied per event.
-// Launches are recorded into a CUDA graph and replayed; tile shape, occupancy,
-// unroll and steps per launch come from an autotuner (vh_batch_autotune).
+// Launches are recorded into a CUDA graph and replayed; blocks per SM and
+// steps per launch come from an autotuner (vh_batch_autotune).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -698,10 +698,11 @@ extern "C" int vh_batch_get_tuning(vh_batch* b, int* variant, int* steps_per_lau
 }
 
 // Autotuner: time `probe_steps` steps of every compiled variant x
-// steps-per-launch choice from the current state (the pool and tables are
-// saved before and restored after each trial), keep the fastest, and cache
-// the choice in cache_path under a key of device, precision and event-size
-// histogram (an existing entry is reused without timing).
+// steps-per-launch choice from the current state (saved before and restored
+// after each trial), keep the fastest, and cache the choice in cache_path
+// under a key of device, precision, event-size histogram, reconstruction, pool
+// layout and the variants' blocks per SM, so that a file of other kernels says
+// nothing here (an existing entry is reused without timing).
 extern "C" int vh_batch_autotune(vh_batch* b, const char* cache_path, int probe_steps, double* best_ms_per_step) {
   if (!b || probe_steps < 1) return VH_E_ARG;
   int dev = 0;
@@ -713,6 +714,9 @@ extern "C" int vh_batch_autotune(vh_batch* b, const char* cache_path, int probe_
   std::ostringstream key;
   key << prop.name << "|" << (b->mixed ? "mixed" : "fp64") << "|" << b->n;
   for (long long h : hist) key << ":" << h;
+  const int* blocks_of = b->mixed ? kBlocks32 : kBlocks64;
+  key << "|recon " << b->cfg.recon << "|arrays " << b->arrays << "|blocks of " << kSweepThreads;
+  for (int v = 0; v < kNumVariants; v++) key << ":" << blocks_of[v];
   if (cache_path) {
     std::ifstream in(cache_path);
     std::string line;
@@ -750,7 +754,8 @@ extern "C" int vh_batch_autotune(vh_batch* b, const char* cache_path, int probe_
   }
   double best = 1e300;
   int best_v = b->variant, best_s = b->steps_per_launch;
-  for (int v = 0; v < kNumVariants; v++)
+  for (int v = 0; v < kNumVariants; v++) {
+    if (std::find(blocks_of, blocks_of + v, blocks_of[v]) != blocks_of + v) continue;  // the same kernel again
     for (int spl : kStepsChoices) {
       int blocks = 0;
       if (launch(b, v, 0, 0, true, &blocks) != VH_OK || blocks <= 0) continue;
@@ -768,6 +773,7 @@ extern "C" int vh_batch_autotune(vh_batch* b, const char* cache_path, int probe_
       const double ms = 1e3 * sec / steps;
       if (ms < best) { best = ms; best_v = v; best_s = spl; }
     }
+  }
   if (!restore()) return VH_E_CUDA;
   cudaFree(save);
   vh_batch_reset(b);
