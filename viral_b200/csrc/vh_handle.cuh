@@ -92,27 +92,6 @@ static constexpr int kStateArrays = 52;
 
 static inline unsigned grid1(long long n, int b) { return (unsigned)((n + b - 1) / b); }
 
-// A step kernel launched with programmatic stream serialization (when pdl):
-// it may begin while the kernel before it in the stream finishes its last
-// blocks; the kernel itself waits for that kernel's completion before
-// reading anything (pdl_wait_then_release), so the overlap covers launch and
-// block set-up.
-template <class K, class... Args>
-static cudaError_t launch_step_kernel(bool pdl, K kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t s,
-                                      Args... args) {
-  cudaLaunchConfig_t lc = {};
-  lc.gridDim = grid;
-  lc.blockDim = block;
-  lc.dynamicSmemBytes = smem;
-  lc.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  lc.attrs = at;
-  lc.numAttrs = pdl ? 1 : 0;
-  return cudaLaunchKernelEx(&lc, kernel, args...);
-}
-
 // The flux sweeps of a stage along directions d0..d1-1, one launch.
 template <class R>
 static int launch_dirs(vh_handle* h, const DevPtrs<R>& P, int d0, int d1, int use_b, double tau) {

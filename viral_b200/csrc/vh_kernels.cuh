@@ -26,6 +26,27 @@ __device__ __forceinline__ void pdl_wait_then_release() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// A step kernel launched with programmatic stream serialization (when pdl):
+// it may begin while the kernel before it in the stream finishes its last
+// blocks; the kernel itself waits for that kernel's completion before
+// reading anything (pdl_wait_then_release), so the overlap covers launch and
+// block set-up.
+template <class K, class... Args>
+static cudaError_t launch_step_kernel(bool pdl, K kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                                      Args... args) {
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = grid;
+  lc.blockDim = block;
+  lc.dynamicSmemBytes = smem;
+  lc.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  lc.attrs = at;
+  lc.numAttrs = pdl ? 1 : 0;
+  return cudaLaunchKernelEx(&lc, kernel, args...);
+}
+
 // The tensor maps of the state: per direction, arrays 0..4 (e, u^mu) and one
 // conserved set (9 arrays); used by the TMA-staged sweeps alone.
 struct alignas(64) TileMaps {

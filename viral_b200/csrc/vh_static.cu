@@ -38,7 +38,7 @@ using namespace vh;
 
 namespace {
 
-constexpr long long kStaticArrays = 34;  // B(9) + v1t(4) + res(9) + du(12)
+constexpr long long kStaticArrays = 34;  // B(9) + v1t(4) + res(9) + du(12), and res along y and eta where they fit
 constexpr long long kStaticCells = VH_STATIC_MAX_CELLS;
 constexpr long long kHeaderDoubles = 32;  // status word and iteration counter
 
@@ -108,16 +108,21 @@ int fill_cfg(const vh_config* c, const double* eos_dev, double tau, DevCfg& C) {
   return VH_OK;
 }
 
-// The sweeps of a stage one direction after the other, each adding to the one
-// divergence array the scratch has room for.
+// The sweeps of a stage: one launch where every direction has a divergence
+// set, else the directions one after the other, each adding to the one set.
 int launch_dirs_static(const DevCfg& C, const DevPtrs<double>& P, const SweepPlan& plan, int use_b, double tau,
                        cudaStream_t s) {
   const TileMaps none{};  // read by the TMA-staged kernels alone
+  auto kern = C.recon != 0 ? k_dir<double, true, false> : k_dir<double, false, false>;
   const int dirs = C.bi ? 2 : 3;
-  for (int d = 0, first = 0; d < dirs; first += plan.blocks(d++)) {
-    auto kern = C.recon != 0 ? k_dir<double, true, false> : k_dir<double, false, false>;
-    kern<<<plan.blocks(d), kSweepThreads, sweep_smem<double>(plan, dirs), s>>>(C, P, use_b, tau, plan, first, none);
-    if (cudaGetLastError() != cudaSuccess) return VH_E_CUDA;
+  for (int d = 0, first = 0; d < dirs;) {
+    int n = 0;
+    do n += plan.blocks(d++);
+    while (P.res1 && d < dirs);
+    if (launch_step_kernel(P.res1 != nullptr, kern, dim3(n), dim3(kSweepThreads), sweep_smem<double>(plan, dirs), s, C,
+                           P, use_b, tau, plan, first, none) != cudaSuccess)
+      return VH_E_CUDA;
+    first += n;
   }
   return VH_OK;
 }
@@ -143,9 +148,15 @@ extern "C" int vh_step_static(const vh_config* cfg, double* state, const double*
   P.stride = n;
   P.status = reinterpret_cast<unsigned int*>(scratch);
   P.iters = reinterpret_cast<unsigned long long*>(scratch + 1);
+  // A divergence set per direction (9 more arrays, 18 in 3+1D) on grids that
+  // leave room for them in the scratch: 4 launches a step, each under the last
+  // blocks of the one before, instead of 6 or 8 (us a step with WENO5: 129x129
+  // 74 to 46, 10x10x41 94 to 50).  Larger grids add up one set in order;
+  // overlapping those launches costs them 5 %.
+  if ((34 + (C.bi ? 9 : 18)) * n <= kStaticArrays * kStaticCells) P.res1 = P.base1 + 34 * n;
   if (cudaMemsetAsync(scratch, 0, kHeaderDoubles * sizeof(double), s) != cudaSuccess) return VH_E_CUDA;
 
-  const SweepPlan plan = sweep_plan<double>(C);
+  const SweepPlan plan = sweep_plan<double>(C, P.res1 != nullptr);
   const double ts = cfg->dtau;
   const long long nint = (long long)C.nx * C.ny * (C.kr - C.kl);
   const unsigned blocks = (unsigned)((nint + kUpdThreads - 1) / kUpdThreads);
@@ -153,9 +164,9 @@ extern "C" int vh_step_static(const vh_config* cfg, double* state, const double*
     for (int stage = 0; stage < 2; stage++) {
       const double t = stage ? tau + ts : tau;
       if (int r = launch_dirs_static(C, P, plan, stage, t, s)) return r;
-      if (stage == 0) k_update<double, 1><<<blocks, kUpdThreads, 0, s>>>(C, P, tau, ts);
-      else k_update<double, 2><<<blocks, kUpdThreads, 0, s>>>(C, P, tau, ts);
-      if (cudaGetLastError() != cudaSuccess) return VH_E_CUDA;
+      if (launch_step_kernel(P.res1 != nullptr, stage == 0 ? k_update<double, 1> : k_update<double, 2>, dim3(blocks),
+                             dim3(kUpdThreads), 0, s, C, P, tau, ts) != cudaSuccess)
+        return VH_E_CUDA;
     }
     tau += ts;
   }

@@ -655,11 +655,17 @@ __device__ __forceinline__ void sweep_tile(const DevCfg& C, const DevPtrs<R>& P,
 // cells: FP64 1.293 / 1.383 / 1.381, FP32 0.808 / 0.802 / 0.802.  Grids with
 // fewer than two such tiles per SM take up to 16 cells, more blocks of less
 // latency (129x129: 0.0543 ms per step at 16, 0.0568 at 24, 0.0556 at 8).
+// Where the directions are launched one by one (together false: the
+// allocation-free step's largest grids, up to 61,680 cells with ghosts) a
+// launch has a third or half of the tiles, and 12 cells are best: 240x240 at
+// 8 / 12 / 16 / 24 cells 102 / 88 / 91 / 104 us a step, 34x34x32 121 / 111 /
+// 116 / 125.
 template <class R>
-static SweepPlan sweep_plan(const DevCfg& C) {
+static SweepPlan sweep_plan(const DevCfg& C, bool together = true) {
   SweepPlan p{};
   const int len[3] = {C.nx, C.ny, C.kr - C.kl}, dirs = C.bi ? 2 : 3;
-  for (int most : {sizeof(R) == 8 ? 24 : 30, 16}) {
+  const int longest = together ? (sizeof(R) == 8 ? 24 : 30) : 12;
+  for (int most : {longest, longest < 16 ? longest : 16}) {
     int tiles = 0;
     for (int d = 0; d < dirs; d++) {
       const int k = (len[d] + most - 1) / most;
