@@ -92,6 +92,12 @@ static constexpr int kStateArrays = 52;
 
 static inline unsigned grid1(long long n, int b) { return (unsigned)((n + b - 1) / b); }
 
+template <class R>
+static auto sweep_kernel(const vh_handle* h, bool tma) {
+  const bool mm = h->C.recon != 0;
+  return tma ? (mm ? k_dir<R, true, true> : k_dir<R, false, true>) : (mm ? k_dir<R, true, false> : k_dir<R, false, false>);
+}
+
 // The flux sweeps of a stage along directions d0..d1-1, one launch.
 template <class R>
 static int launch_dirs(vh_handle* h, const DevPtrs<R>& P, int d0, int d1, int use_b, double tau) {
@@ -99,10 +105,9 @@ static int launch_dirs(vh_handle* h, const DevPtrs<R>& P, int d0, int d1, int us
   const SweepPlan& p = h->plan;
   int first = 0, n = 0;
   for (int d = 0; d < d1; d++) (d < d0 ? first : n) += p.blocks(d);
-  const bool mm = C.recon != 0;
   // one divergence array for all directions (P.res1 null): the cached kernels
-  auto kern = h->tma && P.res1 ? (mm ? k_dir<R, true, true> : k_dir<R, false, true>)
-                     : (mm ? k_dir<R, true, false> : k_dir<R, false, false>);
+  // (a plan's tile stays below the 48 KB that need no attribute)
+  auto kern = sweep_kernel<R>(h, h->tma && P.res1);
   VH_CUDA(h, launch_step_kernel(h->pdl, kern, dim3(n), dim3(kSweepThreads), sweep_smem<R>(p, C.bi ? 2 : 3), h->stream,
                                 C, P, use_b, (R)tau, p, first, h->tmap));
   return VH_OK;
@@ -157,10 +162,8 @@ template <class R>
 static int set_smem_attrs(vh_handle* h) {
   h->plan = sweep_plan<R>(h->C);
   encode_maps<R>(h);
-  VH_CUDA(h, set_sweep_smem(k_dir<R, false, true>));
-  VH_CUDA(h, set_sweep_smem(k_dir<R, true, true>));
-  VH_CUDA(h, set_sweep_smem(k_dir<R, false, false>));
-  VH_CUDA(h, set_sweep_smem(k_dir<R, true, false>));
+  // for the kernel the steps will launch alone: this loads it
+  VH_CUDA(h, set_sweep_smem(sweep_kernel<R>(h, h->tma)));
   return VH_OK;
 }
 
