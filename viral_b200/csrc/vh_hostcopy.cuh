@@ -91,19 +91,30 @@ class HostCopy {
   // dst (any memory) <- src (device), after the work already in `stream`.
   // Pinned, device and small destinations take the runtime's copy, which is
   // in `stream` and may still be under way at return; otherwise dst is
-  // complete at return.
+  // complete at return.  The slots, streams and events are made on src's device
+  // and used there whichever is current (a null stream is the current one's and
+  // takes the threads only where that is src's).
   cudaError_t copy(void* dst, const void* src, size_t bytes, cudaStream_t stream) {
-    cudaPointerAttributes a;
+    cudaPointerAttributes a, from;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    int current = 0;
     const bool plain = bytes >= kLeast && cudaPointerGetAttributes(&a, dst) == cudaSuccess &&
                        a.type == cudaMemoryTypeUnregistered &&
                        cudaStreamIsCapturing(stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone &&
-                       make();
+                       cudaPointerGetAttributes(&from, src) == cudaSuccess && cudaGetDevice(&current) == cudaSuccess &&
+                       (stream || from.device == current);
+    const int dev = plain ? from.device : 0;
+    const bool threaded = plain && cudaSetDevice(dev) == cudaSuccess && make();
     cudaGetLastError();
-    if (!plain) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, stream);
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaEventRecord(ready_, stream);
+    const cudaError_t e = threaded ? by_threads(dst, src, bytes, stream, dev)
+                                   : cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, stream);
+    if (plain && current != dev) cudaSetDevice(current);
+    return e;
+  }
+
+ private:
+  cudaError_t by_threads(void* dst, const void* src, size_t bytes, cudaStream_t stream, int dev) {
+    const cudaError_t e = cudaEventRecord(ready_, stream);
     if (e != cudaSuccess) return e;
     std::atomic<int> err{(int)cudaSuccess};
     // parts of whole pages, so that no two threads fault the same one
