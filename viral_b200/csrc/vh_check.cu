@@ -1,7 +1,10 @@
 // Host-side entry points onto the device arithmetic of the step and of its
 // adjoint (the same __host__ __device__ functions the kernels use), for the
 // CPU tests: finite-difference checks of every local adjoint.  Test hooks
-// only: not part of the C ABI in include/vh.h, built as libvh_check.so.
+// only: not part of the C ABI in include/vh.h, built as libvh_check.so.  The
+// two entries with kernels run what the host's branch does not compile, the
+// reciprocals from the hardware's seeds and the root-find on them.
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -47,9 +50,74 @@ HostCfg make_cfg(const vh_config* c) {
   }
   return h;
 }
+
+// out, 7 rows of n: fast_rcp, rcp_any and the two roots of x in FP64; of (float)x
+// fast_rcp, rcp and rcp_any.  ref, 3 rows: CUDA's 1/x, sqrt(x) and 1/sqrt(x)
+__global__ void k_seeds(const double* x, long long n, double* out, double* ref) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double v = x[i];
+  const float f = (float)v;
+  double root, inv;
+  root_rsqrt(v, root, inv);
+  out[i] = fast_rcp(v);
+  out[n + i] = rcp_any<double>(v);
+  out[2 * n + i] = root;
+  out[3 * n + i] = inv;
+  out[4 * n + i] = fast_rcp(f);
+  out[5 * n + i] = rcp<float>(f);
+  out[6 * n + i] = rcp_any<float>(f);
+  ref[i] = 1.0 / v;
+  ref[n + i] = sqrt(v);
+  ref[2 * n + i] = 1.0 / sqrt(v);
+}
+__global__ void k_con2prim(DevCfg C, long long n, const double* T, const double* p, double tau, double* x, int* it) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  it[i] = con2prim(C, T + 4 * i, p + 5 * i, tau, x + 4 * i);
+}
+// memory on both sides, gone with the object
+template <class T>
+struct Shared {
+  T* p = nullptr;
+  explicit Shared(size_t n) {
+    if (cudaMallocManaged(&p, n * sizeof(T)) != cudaSuccess) p = nullptr;
+  }
+  ~Shared() { cudaFree(p); }
+};
 }  // namespace
 
 extern "C" {
+
+int vhc_seeds_gpu(const double* x, long long n, double* out7, double* ref3) {
+  Shared<double> b(11 * n);
+  if (!b.p) return VH_E_NOMEM;
+  std::copy(x, x + n, b.p);
+  k_seeds<<<(unsigned)((n + 255) / 256), 256>>>(b.p, n, b.p + n, b.p + 8 * n);
+  if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) return VH_E_CUDA;
+  std::copy(b.p + n, b.p + 8 * n, out7);
+  std::copy(b.p + 8 * n, b.p + 11 * n, ref3);
+  return VH_OK;
+}
+// vhc_con2prim4 of n cells on the GPU: T 4, p 5, x 4 words a cell
+int vhc_con2prim4_gpu(const vh_config* c, long long n, const double* T, const double* p, double tau, double* x,
+                      int* it) {
+  HostCfg h = make_cfg(c);
+  Shared<double> b(13 * n + h.td.size());
+  Shared<int> k(n);
+  if (!b.p || !k.p) return VH_E_NOMEM;
+  double *bT = b.p, *bp = bT + 4 * n, *bx = bp + 5 * n, *tab = bx + 4 * n;
+  std::copy(T, T + 4 * n, bT);
+  std::copy(p, p + 5 * n, bp);
+  std::copy(x, x + 4 * n, bx);
+  std::copy(h.td.begin(), h.td.end(), tab);
+  h.C.eos_d = tab;
+  k_con2prim<<<(unsigned)((n + 127) / 128), 128>>>(h.C, n, bT, bp, tau, bx, k.p);
+  if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) return VH_E_CUDA;
+  std::copy(bx, bx + 4 * n, x);
+  std::copy(k.p, k.p + n, it);
+  return VH_OK;
+}
 
 void vhc_weno_lr(const double* q, double* L, double* R) { weno_lr<double>(q[0], q[1], q[2], q[3], q[4], *L, *R); }
 void vhc_weno_lr_vjp(const double* q, double Lb, double Rb, double* qb) { weno_lr_vjp<double>(q, Lb, Rb, qb); }

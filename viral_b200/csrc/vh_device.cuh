@@ -84,13 +84,13 @@ __host__ VH_HD inline long long cix(const DevCfg& C, int i, int j, int k) {
 
 // ---------------------------------------------------- reciprocal and root
 // On the device, from the hardware's approximate seeds and one step of an
-// iteration for the zero of 1/r - x or 1/y^2 - s, without the general
-// division's treatment of subnormal and overflowing operands (no operand here
-// comes near them; rcp_any takes those that may be zero or infinite).  On the
-// host, the plain operations.
+// iteration, without the general division's treatment of subnormal and
+// overflowing operands (no operand here comes near them; rcp_any takes those
+// that may be zero or infinite).  On the host, the plain operations.
 //
-// fast_rcp: FP64, the seed (rcp.approx.ftz.f64, about 20 bits) and one
-// third-order step r (1 + d + d^2), d = 1 - x r: the error left is d^3, below
+// fast_rcp: FP64, the seed (rcp.approx.ftz.f64, about 20 bits) and one step of
+// the hyperpower iteration of order three (Altman 1960), r (1 + d + d^2) with
+// d = 1 - x r: of the geometric series of 1/(1 - d) the step leaves d^3, below
 // the last bit.  FP32, the seed alone (1 ulp).
 #ifdef __CUDACC__
 __device__ __forceinline__ double fast_rcp(double x) {
@@ -133,9 +133,11 @@ VH_HD inline R rcp_any(R x) {
   return (R)1 / x;
 #endif
 }
-// sqrt(s) and 1/sqrt(s) of s >= 1: the seed (rsqrt.approx.ftz.f64), one
-// third-order step y (1 + d/2 + 3 d^2/8), d = 1 - s y^2, and a Newton
-// correction of the root
+// sqrt(s) and 1/sqrt(s) of s >= 1: the seed (rsqrt.approx.ftz.f64), one step
+// of Chebyshev's iteration for 1/y^2 = s, y (1 + d/2 + 3 d^2/8) with
+// d = 1 - s y^2 (the binomial series of (1 - d)^(-1/2), 5 d^3/16 left), and for
+// the root Heron's correction r + (s - r^2)/(2 r).  The root is within an ulp,
+// its reciprocal within 5/4 (the rounding of s y enters it by half).
 VH_HD inline void root_rsqrt(double s, double& root, double& inv) {
 #ifdef __CUDA_ARCH__
   double y;
@@ -611,8 +613,12 @@ VH_HD inline bool solve4(double A[4][4], double b[4]) {
 // entry and candidate (a third of the update kernel's instructions were
 // theirs): false, with A and b spoilt, where a multiplier exceeds 1024 and
 // the exchange is worth having.  The Jacobian is dominated by its diagonal at
-// ordinary velocities; multipliers below 1024 leave a Newton step 1e-7 of its
-// length uncertain at the very worst, and the last step is below 1e-8.
+// ordinary velocities.  Multipliers below 1024 let the elimination's rounding
+// grow to 1024^3 units, 1e-7 of the matrix; a step's relative error is that
+// times the Jacobian's condition number.  The loop evaluates the residual at
+// the end of such a step and shortens one that does not reduce it.  The last
+// step may go without (con2prim's qskip): it is below 1e-8 of x, and so is its
+// error up to a condition number of 1e7.
 VH_HD inline bool solve4_direct(double A[4][4], double b[4]) {
   bool ok = true;
 #pragma unroll

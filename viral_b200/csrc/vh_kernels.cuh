@@ -378,8 +378,8 @@ __device__ __forceinline__ unsigned update_cell(const DevCfg& C, const DevPtrs<R
 }
 
 // One thread per interior cell.  Bound by the latency of its loads and of the
-// Newton chain, with DRAM at half its rate (88 words a cell and launch in
-// 3+1D).  Blocks per SM: FP64 4 (128 registers), mixed 5 (96); measured on the
+// Newton chain, with DRAM at half its rate (79 words a cell at
+// stage 1 and 84 at stage 2 in 3+1D).  Blocks per SM: FP64 4 (128 registers), mixed 5 (96); measured on the
 // 161x161x41 event, ms per stage-1 launch: FP64 0.220 / 0.213 / 0.305 at 3 / 4 /
 // 5 blocks (spills), mixed 0.155 / 0.146 / 0.145 at 4 / 5 / 6.  Divisions and
 // roots by the hardware's seeds and one step (rcp, root_rsqrt), elimination

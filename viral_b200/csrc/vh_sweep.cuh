@@ -359,8 +359,9 @@ __device__ __forceinline__ void walk(const DevPtrs<R>& P, const SweepLay<R, DIR>
       v_split(f.nr, m0, m1);
       v_split(f.sr, r0, r1);
       if constexpr (sizeof(R) == 8) {
-        // one reciprocal for the face's four quotients (the product of the
-        // sums stays far inside double range)
+        // one reciprocal for the face's four quotients.  A sum lies between
+        // 1e-23 (the weights' eps alone) and 1.3e7 |q|^8: up to |q| = 1e8 the
+        // products of four and of their numerators are inside double range
         R s0, s1;
         v_split(slp, s0, s1);
         const R nf = fma(n0, r0, m0 * s0), nv = am * fma(n1, r1, -(m1 * s1)), df = s0 * r0, dv = s1 * r1;
