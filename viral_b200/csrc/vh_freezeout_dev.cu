@@ -183,6 +183,30 @@ __global__ void __launch_bounds__(kCfThreads, 4) k_cooper_frye(const double* __r
       part[((long long)blockIdx.x * kBins + tid / 32 * kWarpBins + b) * gridDim.y + blockIdx.y] = acc[b];
   }
 }
+// The same for tiles of one bin, a thread an element with all of the bin's
+// term: in 2+1D with a single azimuth nothing of an element is shared between
+// bins, and the Bessel functions, which bound it, want the warps that an
+// accumulator and no staging leave room for.  0.8 M elements and 400 x 1 bins:
+// 54.3 ms as tiles of 16, 46.0 with the missing bins left out of them, 34.9 so,
+// and 37.8 a bin a block over all elements (with two azimuths 69.8 a bin a
+// block, 54.3 as tiles).
+__global__ void __launch_bounds__(kThreads) k_cooper_frye_one(const double* __restrict__ el, long long count,
+                                                              const double* __restrict__ bins, double t_fo,
+                                                              double* __restrict__ part) {
+  __shared__ double red[kThreads / 32];
+  const int tid = threadIdx.x;
+  const double* m = bins + (long long)blockIdx.x * kBins * 3;
+  const double mt = m[0], px = m[1], py = m[2];
+  double s = 0;
+  for (long long e = (long long)blockIdx.y * kThreads + tid; e < count; e += (long long)gridDim.y * kThreads)
+    s += vh_fo::cf2_term(el + vh_fo::kW2 * e, mt, px, py, t_fo);
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if (tid % 32 == 0) red[tid / 32] = s;
+  __syncthreads();
+  if (tid) return;
+  for (int w = 1; w < kThreads / 32; w++) s += red[w];
+  part[(long long)blockIdx.x * kBins * gridDim.y + blockIdx.y] = s;
+}
 // the shares' sums, one warp per slot; slot q of tile t is the bin
 // first_bin(t) + q of the spectrum
 struct CfTiles {
@@ -274,9 +298,12 @@ int spectrum(const double* el, long long count, double t_fo, double mass, double
   const CfTiles tl{nphi, D == 3 ? (nphi + kBins - 1) / kBins : 0, nb};
   const long long tiles = D == 3 ? (long long)npt * tl.per_row : (nb + kBins - 1) / kBins;
   const int chunk = (int)(tiles < kMostTiles ? tiles : kMostTiles);
-  // shares of the elements: about four blocks per SM over the tiles
-  const long long most = (count + kCfThreads - 1) / kCfThreads;
-  long long shares = (4 * 148 + chunk - 1) / chunk;
+  const bool one = D == 3 && nphi == 1;
+  // shares of the elements: about four blocks per SM over the tiles (eight of
+  // single bins)
+  const int threads = one ? kThreads : kCfThreads;
+  const long long most = (count + threads - 1) / threads;
+  long long shares = ((one ? 8 : 4) * 148 + chunk - 1) / chunk;
   shares = shares > most ? most : shares;
   shares = shares < 1 ? 1 : shares;
   std::vector<double> bins(3 * kBins * (size_t)tiles, 0.0);
@@ -304,7 +331,9 @@ int spectrum(const double* el, long long count, double t_fo, double mass, double
       rc = VH_E_CUDA;
       break;
     }
-    k_cooper_frye<D><<<dim3((unsigned)n, (unsigned)shares), kCfThreads, 0, st>>>(el, count, dbuf, y, t_fo, part);
+    const dim3 grid((unsigned)n, (unsigned)shares);
+    if (one) k_cooper_frye_one<<<grid, kThreads, 0, st>>>(el, count, dbuf, t_fo, part);
+    else k_cooper_frye<D><<<grid, kCfThreads, 0, st>>>(el, count, dbuf, y, t_fo, part);
     k_cf_final<<<(unsigned)(((long long)n * kBins * 32 + 255) / 256), 256, 0, st>>>(part, (int)shares, tl, t0, n, pref,
                                                                                     dout);
     if (cudaGetLastError() != cudaSuccess) rc = VH_E_CUDA;
