@@ -9,6 +9,7 @@
 // momentum bin in a fixed order (deterministic).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <climits>
 #include <cmath>
 #include <vector>
@@ -299,13 +300,16 @@ int spectrum(const double* el, long long count, double t_fo, double mass, double
   const long long tiles = D == 3 ? (long long)npt * tl.per_row : (nb + kBins - 1) / kBins;
   const int chunk = (int)(tiles < kMostTiles ? tiles : kMostTiles);
   const bool one = D == 3 && nphi == 1;
-  // shares of the elements: about four blocks per SM over the tiles (eight of
-  // single bins)
+  // shares of the elements: about four blocks per SM over the launch's tiles
+  // (eight of single bins)
   const int threads = one ? kThreads : kCfThreads;
   const long long most = (count + threads - 1) / threads;
-  long long shares = ((one ? 8 : 4) * 148 + chunk - 1) / chunk;
-  shares = shares > most ? most : shares;
-  shares = shares < 1 ? 1 : shares;
+  auto shares_of = [&](long long n) {
+    const long long k = ((one ? 8 : 4) * 148 + n - 1) / n;
+    return k > most ? (most < 1 ? 1 : most) : k;
+  };
+  const long long last = tiles % chunk;  // tiles of a shorter last launch
+  const long long parts = std::max(chunk * shares_of(chunk), last ? last * shares_of(last) : 0);
   std::vector<double> bins(3 * kBins * (size_t)tiles, 0.0);
   for (long long t = 0; t < tiles; t++)
     for (long long i = tl.first(t); i < tl.end(t); i++) {
@@ -315,7 +319,7 @@ int spectrum(const double* el, long long count, double t_fo, double mass, double
       q[1] = p * std::cos(f);
       q[2] = p * std::sin(f);
     }
-  const size_t w_bins = 3 * kBins * (size_t)chunk, w_part = (size_t)(chunk * kBins * shares);
+  const size_t w_bins = 3 * kBins * (size_t)chunk, w_part = (size_t)(kBins * parts);
   double* dbuf = nullptr;
   if (cudaMallocAsync((void**)&dbuf, (w_bins + w_part + (size_t)nb) * sizeof(double), st) != cudaSuccess) {
     cudaGetLastError();
@@ -331,11 +335,11 @@ int spectrum(const double* el, long long count, double t_fo, double mass, double
       rc = VH_E_CUDA;
       break;
     }
+    const int shares = (int)shares_of(n);
     const dim3 grid((unsigned)n, (unsigned)shares);
     if (one) k_cooper_frye_one<<<grid, kThreads, 0, st>>>(el, count, dbuf, t_fo, part);
     else k_cooper_frye<D><<<grid, kCfThreads, 0, st>>>(el, count, dbuf, y, t_fo, part);
-    k_cf_final<<<(unsigned)(((long long)n * kBins * 32 + 255) / 256), 256, 0, st>>>(part, (int)shares, tl, t0, n, pref,
-                                                                                    dout);
+    k_cf_final<<<(unsigned)(((long long)n * kBins * 32 + 255) / 256), 256, 0, st>>>(part, shares, tl, t0, n, pref, dout);
     if (cudaGetLastError() != cudaSuccess) rc = VH_E_CUDA;
   }
   if (rc == VH_OK &&
