@@ -1,6 +1,8 @@
 """Spectra with few azimuths a p_T, which a block's warps share by elements
 instead of by bins, and with tiles of every number of bins: against the host
 sums."""
+import resource
+
 import numpy as np
 import pytest
 
@@ -30,3 +32,19 @@ def test_tiles_of_few_bins(nphi, count):
         host = host_fn(el, 0.15, 0.7, 3.0, *rap, pt, phi)
         got = dev_fn(dev(el), 0.15, 0.7, 3.0, *rap, pt, phi)
         assert np.allclose(got, host, rtol=1e-12, atol=0)
+
+
+def test_host_memory_of_many_bins():
+    """A million p_T at one azimuth: the call's host scratch is that of one
+    launch's bins, well below 100 MB more than the bins and results in hand
+    (in tiles of 16 all bins took 384 MB)."""
+    npt = 1_000_000
+    pt, phi = np.linspace(0.1, 2.0, npt), np.zeros(1)
+    el = np.array([[1.0, 0, 0, 1.0, 0.1, 0.1, 1.0, 0, 0]])
+    cooper_frye_2d_device(dev(el), 0.15, 0.7, 3.0, pt[:1000], phi)
+    before = resource.getrusage(resource.RUSAGE_SELF).ru_maxrss
+    got = cooper_frye_2d_device(dev(el), 0.15, 0.7, 3.0, pt, phi)
+    grown = resource.getrusage(resource.RUSAGE_SELF).ru_maxrss - before
+    pick = slice(0, npt, 9973)
+    assert np.allclose(got[pick], cooper_frye_2d(el, 0.15, 0.7, 3.0, pt[pick], phi), rtol=1e-12, atol=0)
+    assert grown < 100_000  # KB

@@ -310,15 +310,7 @@ int spectrum(const double* el, long long count, double t_fo, double mass, double
   };
   const long long last = tiles % chunk;  // tiles of a shorter last launch
   const long long parts = std::max(chunk * shares_of(chunk), last ? last * shares_of(last) : 0);
-  std::vector<double> bins(3 * kBins * (size_t)tiles, 0.0);
-  for (long long t = 0; t < tiles; t++)
-    for (long long i = tl.first(t); i < tl.end(t); i++) {
-      double* q = &bins[3 * (size_t)(t * kBins + i - tl.first(t))];
-      const double p = pt[i / nphi], f = phi[i % nphi];
-      q[0] = std::sqrt(mass * mass + p * p);
-      q[1] = p * std::cos(f);
-      q[2] = p * std::sin(f);
-    }
+  std::vector<double> bins(3 * kBins * (size_t)chunk);  // of one launch
   const size_t w_bins = 3 * kBins * (size_t)chunk, w_part = (size_t)(kBins * parts);
   double* dbuf = nullptr;
   if (cudaMallocAsync((void**)&dbuf, (w_bins + w_part + (size_t)nb) * sizeof(double), st) != cudaSuccess) {
@@ -330,7 +322,17 @@ int spectrum(const double* el, long long count, double t_fo, double mass, double
   int rc = VH_OK;
   for (long long t0 = 0; t0 < tiles && rc == VH_OK; t0 += chunk) {
     const int n = (int)(tiles - t0 < chunk ? tiles - t0 : chunk);
-    if (cudaMemcpyAsync(dbuf, &bins[3 * kBins * (size_t)t0], 3 * kBins * (size_t)n * sizeof(double),
+    std::fill(bins.begin(), bins.end(), 0.0);
+    for (long long t = t0; t < t0 + n; t++)
+      for (long long i = tl.first(t); i < tl.end(t); i++) {
+        double* q = &bins[3 * (size_t)((t - t0) * kBins + i - tl.first(t))];
+        const double p = pt[i / nphi], f = phi[i % nphi];
+        q[0] = std::sqrt(mass * mass + p * p);
+        q[1] = p * std::cos(f);
+        q[2] = p * std::sin(f);
+      }
+    // (from pageable memory: staged when the call returns)
+    if (cudaMemcpyAsync(dbuf, bins.data(), 3 * kBins * (size_t)n * sizeof(double),
                         cudaMemcpyHostToDevice, st) != cudaSuccess) {
       rc = VH_E_CUDA;
       break;
