@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(kThreads) k_cooper_frye_one(const double* __re
                                                               double* __restrict__ part) {
   __shared__ double red[kThreads / 32];
   const int tid = threadIdx.x;
-  const double* m = bins + (long long)blockIdx.x * kBins * 3;
+  const double* m = bins + (long long)blockIdx.x * 3;
   const double mt = m[0], px = m[1], py = m[2];
   double s = 0;
   for (long long e = (long long)blockIdx.y * kThreads + tid; e < count; e += (long long)gridDim.y * kThreads)
@@ -206,18 +206,18 @@ __global__ void __launch_bounds__(kThreads) k_cooper_frye_one(const double* __re
   __syncthreads();
   if (tid) return;
   for (int w = 1; w < kThreads / 32; w++) s += red[w];
-  part[(long long)blockIdx.x * kBins * gridDim.y + blockIdx.y] = s;
+  part[(long long)blockIdx.x * gridDim.y + blockIdx.y] = s;
 }
 // the shares' sums, one warp per slot; slot q of tile t is the bin
 // first_bin(t) + q of the spectrum
 struct CfTiles {
-  int nphi, per_row;  // per_row: tiles of a p_T (2+1D), 0: tiles run on over the bins (3+1D)
+  int nphi, width, per_row;  // per_row: tiles of a p_T (2+1D), 0: tiles run on over the bins (3+1D)
   long long nb;
   __host__ __device__ long long first(long long t) const {
-    return per_row ? t / per_row * nphi + t % per_row * kBins : t * kBins;
+    return per_row ? t / per_row * nphi + t % per_row * width : t * width;
   }
   __host__ __device__ long long end(long long t) const {
-    const long long f = first(t) + kBins, m = per_row ? (t / per_row + 1) * nphi : nb;
+    const long long f = first(t) + width, m = per_row ? (t / per_row + 1) * nphi : nb;
     return f < m ? f : m;
   }
 };
@@ -225,8 +225,8 @@ __global__ void k_cf_final(const double* __restrict__ part, int shares, CfTiles 
                            double pref, double* __restrict__ out) {
   const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / 32;
   const int lane = threadIdx.x & 31;
-  if (w >= (long long)tiles * kBins) return;
-  const long long t = tile0 + w / kBins, bin = tl.first(t) + w % kBins;
+  if (w >= (long long)tiles * tl.width) return;
+  const long long t = tile0 + w / tl.width, bin = tl.first(t) + w % tl.width;
   if (bin >= tl.end(t)) return;
   double s = 0;
   for (int k = lane; k < shares; k += 32) s += part[w * shares + k];
@@ -292,14 +292,15 @@ int spectrum(const double* el, long long count, double t_fo, double mass, double
   const long long nb = (long long)npt * nphi;
   if (nb > INT_MAX) return VH_E_ARG;
   VhNvtxRange range("Cooper-Frye spectrum");
-  // bins in tiles of kBins: in 2+1D the azimuths of one p_T (the Bessel
-  // functions depend on p_T alone), in 3+1D any; kMostTiles tiles a launch,
-  // which bounds the scratch
-  constexpr long long kMostTiles = 1024;
-  const CfTiles tl{nphi, D == 3 ? (nphi + kBins - 1) / kBins : 0, nb};
-  const long long tiles = D == 3 ? (long long)npt * tl.per_row : (nb + kBins - 1) / kBins;
-  const int chunk = (int)(tiles < kMostTiles ? tiles : kMostTiles);
+  // bins in tiles of kBins, in 2+1D the azimuths of one p_T (the Bessel
+  // functions depend on p_T alone), of 1 where that is one; in 3+1D any.  A
+  // launch holds 1024 x kBins bins at most, which bounds the scratch
   const bool one = D == 3 && nphi == 1;
+  const int width = one ? 1 : kBins;
+  const long long most_tiles = 1024 * kBins / width;
+  const CfTiles tl{nphi, width, D == 3 ? (nphi + width - 1) / width : 0, nb};
+  const long long tiles = D == 3 ? (long long)npt * tl.per_row : (nb + width - 1) / width;
+  const int chunk = (int)(tiles < most_tiles ? tiles : most_tiles);
   // shares of the elements: about four blocks per SM over the launch's tiles
   // (eight of single bins)
   const int threads = one ? kThreads : kCfThreads;
@@ -310,8 +311,8 @@ int spectrum(const double* el, long long count, double t_fo, double mass, double
   };
   const long long last = tiles % chunk;  // tiles of a shorter last launch
   const long long parts = std::max(chunk * shares_of(chunk), last ? last * shares_of(last) : 0);
-  std::vector<double> bins(3 * kBins * (size_t)chunk);  // of one launch
-  const size_t w_bins = 3 * kBins * (size_t)chunk, w_part = (size_t)(kBins * parts);
+  std::vector<double> bins(3 * width * (size_t)chunk);  // of one launch
+  const size_t w_bins = 3 * width * (size_t)chunk, w_part = (size_t)(width * parts);
   double* dbuf = nullptr;
   if (cudaMallocAsync((void**)&dbuf, (w_bins + w_part + (size_t)nb) * sizeof(double), st) != cudaSuccess) {
     cudaGetLastError();
@@ -325,14 +326,14 @@ int spectrum(const double* el, long long count, double t_fo, double mass, double
     std::fill(bins.begin(), bins.end(), 0.0);
     for (long long t = t0; t < t0 + n; t++)
       for (long long i = tl.first(t); i < tl.end(t); i++) {
-        double* q = &bins[3 * (size_t)((t - t0) * kBins + i - tl.first(t))];
+        double* q = &bins[3 * (size_t)((t - t0) * width + i - tl.first(t))];
         const double p = pt[i / nphi], f = phi[i % nphi];
         q[0] = std::sqrt(mass * mass + p * p);
         q[1] = p * std::cos(f);
         q[2] = p * std::sin(f);
       }
     // (from pageable memory: staged when the call returns)
-    if (cudaMemcpyAsync(dbuf, bins.data(), 3 * kBins * (size_t)n * sizeof(double),
+    if (cudaMemcpyAsync(dbuf, bins.data(), 3 * width * (size_t)n * sizeof(double),
                         cudaMemcpyHostToDevice, st) != cudaSuccess) {
       rc = VH_E_CUDA;
       break;
@@ -341,7 +342,7 @@ int spectrum(const double* el, long long count, double t_fo, double mass, double
     const dim3 grid((unsigned)n, (unsigned)shares);
     if (one) k_cooper_frye_one<<<grid, kThreads, 0, st>>>(el, count, dbuf, t_fo, part);
     else k_cooper_frye<D><<<grid, kCfThreads, 0, st>>>(el, count, dbuf, y, t_fo, part);
-    k_cf_final<<<(unsigned)(((long long)n * kBins * 32 + 255) / 256), 256, 0, st>>>(part, shares, tl, t0, n, pref, dout);
+    k_cf_final<<<(unsigned)(((long long)n * width * 32 + 255) / 256), 256, 0, st>>>(part, shares, tl, t0, n, pref, dout);
     if (cudaGetLastError() != cudaSuccess) rc = VH_E_CUDA;
   }
   if (rc == VH_OK &&
