@@ -381,25 +381,25 @@ def algorithmic_bytes(cfg, kernel: str) -> float:
 
 
 # DRAM bytes (read + write) per interior cell and launch, from one ncu capture
-# of the 121x121x31 case of the bench event (profiles/step_kernels_*.md for the
+# of the bench event at 121x121x31 (profiles/step_kernels_*.md for the
 # sweeps, profiles/update_kernel_*.md for the updates), scaled to a full launch
 # by the cells processed
 MEASURED_TRAFFIC_PER_CELL = {
-    ("fp64", "k_dir_x"): 136.0, ("fp64", "k_dir_y"): 154.0, ("fp64", "k_dir_eta"): 180.0,
+    ("fp64", "k_dir_x"): 136.0, ("fp64", "k_dir_y"): 154.0, ("fp64", "k_dir_eta"): 179.0,
     ("fp64", "k_update_stage1"): 634.0, ("fp64", "k_update_stage2"): 669.0,
-    ("mixed", "k_dir_x"): 66.0, ("mixed", "k_dir_y"): 66.0, ("mixed", "k_dir_eta"): 75.0,
-    ("mixed", "k_update_stage1"): 293.0, ("mixed", "k_update_stage2"): 320.0,
+    ("mixed", "k_dir_x"): 66.0, ("mixed", "k_dir_y"): 67.0, ("mixed", "k_dir_eta"): 77.0,
+    ("mixed", "k_update_stage1"): 289.0, ("mixed", "k_update_stage2"): 318.0,
 }
 
 
 # the bound that does hold for the step kernels: the share of peak of the
 # pipe or issue rate that limits each, from the same ncu captures
 MEASURED_COMPUTE_BOUND = {
-    ("fp64", "k_dir_x"): ("fp64 pipe", 0.544), ("fp64", "k_dir_y"): ("fp64 pipe", 0.557),
-    ("fp64", "k_dir_eta"): ("fp64 pipe", 0.566), ("fp64", "k_update_stage1"): ("issue", 0.352),
-    ("fp64", "k_update_stage2"): ("issue", 0.364),
-    ("mixed", "k_dir_x"): ("issue", 0.588), ("mixed", "k_dir_y"): ("issue", 0.579),
-    ("mixed", "k_dir_eta"): ("issue", 0.641), ("mixed", "k_update_stage1"): ("issue", 0.447),
+    ("fp64", "k_dir_x"): ("fp64 pipe", 0.547), ("fp64", "k_dir_y"): ("fp64 pipe", 0.561),
+    ("fp64", "k_dir_eta"): ("fp64 pipe", 0.564), ("fp64", "k_update_stage1"): ("issue", 0.354),
+    ("fp64", "k_update_stage2"): ("issue", 0.359),
+    ("mixed", "k_dir_x"): ("issue", 0.586), ("mixed", "k_dir_y"): ("issue", 0.586),
+    ("mixed", "k_dir_eta"): ("issue", 0.641), ("mixed", "k_update_stage1"): ("issue", 0.442),
     ("mixed", "k_update_stage2"): ("issue", 0.450),
 }
 
